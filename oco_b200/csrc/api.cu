@@ -792,7 +792,7 @@ int stage_experts(oco_moe_plan* plan, const uint16_t* x, const uint32_t* ids, in
             launch_route_plan(plan, ids, R, E, kBatchCols, rs, st);
             const int groups = (int)batch_max_groups((size_t)R, (size_t)E);
             mark(plan, st, "fragments");
-            batch_fragments_kernel<<<groups, 256, 0, st>>>(x, ws.tiles, ws.tile_count, ws.offsets, ws.route_of_row, per_row,
+            batch_fragments_kernel<FMT><<<groups, 256, 0, st>>>(x, ws.tiles, ws.tile_count, ws.offsets, ws.route_of_row, per_row,
                                                            H, reinterpret_cast<uint4*>(ws.bfrag_in));
             plan->launches += 1;
             const int parts = std::max(1, std::min(8, (4 * plan->sm_count + groups - 1) / groups));

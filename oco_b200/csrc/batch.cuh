@@ -26,15 +26,16 @@ __host__ __device__ inline size_t batch_smem_bytes(int nkb) {
            (size_t)kBatchWarps * 2 * kStageBytes + 16;
 }
 
-// Position (in halves) of element k of column `col` in a group's fragments:
-// frag[((kb * 8 + col) * 4 + tig) * 4 + slot] is a half2 (element 4*tig+slot, element 4*tig+slot+16).
-__host__ __device__ inline size_t batch_frag_pos(int k, int col) {
-    const int kb = k >> 5, j = k & 31, jj = j & 15, sel = j >> 4, tig = jj >> 2, slot = jj & 3;
-    return ((((size_t)kb * kBatchCols + col) * 4 + tig) * 4 + slot) * 2 + sel;
+// Position (in halves) of element k of column `col` in a group's fragments (frag_place within the block).
+__host__ __device__ inline size_t batch_frag_pos(int fmt, int k, int col) {
+    int tig, slot, sel;
+    frag_place(fmt, k & 31, tig, slot, sel);
+    return ((((size_t)(k >> 5) * kBatchCols + col) * 4 + tig) * 4 + slot) * 2 + sel;
 }
 
 // The token rows of every route group as B fragments (bf16 -> half, zero in unused columns).
 // grid: max groups; one thread per 16-byte fragment piece (block, column, tig).
+template <int FMT>
 __global__ void __launch_bounds__(256) batch_fragments_kernel(const uint16_t* __restrict__ x,
                                                               const uint32_t* __restrict__ tiles,
                                                               const uint32_t* __restrict__ tile_count,
@@ -58,10 +59,17 @@ __global__ void __launch_bounds__(256) batch_fragments_kernel(const uint16_t* __
                 __half2 h = __floats2half2_rn(__uint_as_float(a << 16), __uint_as_float(b << 16));
                 return *reinterpret_cast<uint32_t*>(&h);
             };
-            v.x = pair(lo.x & 0xffffu, hi.x & 0xffffu);
-            v.y = pair(lo.x >> 16, hi.x >> 16);
-            v.z = pair(lo.y & 0xffffu, hi.y & 0xffffu);
-            v.w = pair(lo.y >> 16, hi.y >> 16);
+            if (FMT == OCO_FMT_Q4_0) {                        // elements two apart (frag_place)
+                v.x = pair(lo.x & 0xffffu, lo.y & 0xffffu);
+                v.y = pair(lo.x >> 16, lo.y >> 16);
+                v.z = pair(hi.x & 0xffffu, hi.y & 0xffffu);
+                v.w = pair(hi.x >> 16, hi.y >> 16);
+            } else {
+                v.x = pair(lo.x & 0xffffu, hi.x & 0xffffu);
+                v.y = pair(lo.x >> 16, hi.x >> 16);
+                v.z = pair(lo.y & 0xffffu, hi.y & 0xffffu);
+                v.w = pair(lo.y >> 16, hi.y >> 16);
+            }
         }
         out[i] = v;
     }
@@ -149,7 +157,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_rows_kernel(const Batc
                 p.out[(size_t)orow * p.n_out + f] = h;
             } else {
                 p.out[(size_t)orow * p.n_out + operand_pos(FMT, f)] = h;
-                reinterpret_cast<uint16_t*>(fout)[batch_frag_pos(f, col)] = h;
+                reinterpret_cast<uint16_t*>(fout)[batch_frag_pos(FMT, f, col)] = h;
             }
         };
         if (GATED) {

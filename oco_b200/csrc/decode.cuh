@@ -57,6 +57,19 @@ __host__ __device__ constexpr uint32_t frag_region_bytes(int fmt, int nkb) {
 }
 constexpr int kFragBlockBytes = 128;                // B fragments of one block: 2 columns x 4 lanes x 16 bytes
 
+// Where element j of a 32-element block sits in a column's B fragment: half `sel` of slot `slot` of lane `tig`,
+// so that it meets the code of the same element as the format's decoder delivers it: MXFP4 (j, j + 16) of a code
+// byte; Q4_0 elements two apart; Q4_K elements 8 tig .. 8 tig + 7 to lane tig, two apart in fours.
+__host__ __device__ __forceinline__ void frag_place(int fmt, int j, int& tig, int& slot, int& sel) {
+    if (fmt == OCO_FMT_Q4_K) {
+        const int r = j & 7;
+        tig = j >> 3; slot = (r >> 2) * 2 + (r & 1); sel = (r >> 1) & 1;
+        return;
+    }
+    tig = (j & 15) >> 2; slot = j & 3; sel = j >> 4;
+    if (fmt == OCO_FMT_Q4_0) { const int r = slot; slot = (r & 1) + 2 * sel; sel = r >> 1; }
+}
+
 // D = A * B with a zero accumulator, then D += A * B (fp32 accumulate, half operands).
 __device__ __forceinline__ void mma16816_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                uint32_t b0, uint32_t b1) {
@@ -126,14 +139,25 @@ struct Block32<OCO_FMT_Q4_0> {
         return lds8(base, block) | (lds8(base, block + 1) << 8);
     }
     __device__ static __forceinline__ float scale_f32(uint32_t bits) { return f16_bits_to_f32((uint16_t)bits); }
-    __device__ static __forceinline__ uint32_t pair(uint32_t byte) {
-        // 0x6400 | q is the half 1024 + q; subtracting 1032 leaves q - 8 exactly.
-        uint32_t v = (byte & 0xfu) | ((byte & 0xf0u) << 12) | 0x64006400u;
-        __half2 h = __hsub2(*reinterpret_cast<__half2*>(&v), __half2half2(__ushort_as_half((unsigned short)0x6408)));
-        return *reinterpret_cast<uint32_t*>(&h);
-    }
+    // 0x6400 | q is the half 1024 + q and 0x6400 | 16 q is 1024 + 16 q: nibbles 16 bits apart share a half2 where
+    // they stand (one mask-and-set each, one shift for the odd bytes), and q - 8 follows exactly with one half2
+    // operation off the integer pipe, which is what bounds these kernels. The pairs are (e0, e2), (e1, e3) and the
+    // same of the elements 16 further; frag_place() lays the activations out to match.
+    // Against a shift and two masks per code byte: one Nemotron-H token 55.8 -> 49.7 us.
     __device__ static __forceinline__ void quads(uint32_t w, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-        r0 = pair(w); r1 = pair(w >> 8); r2 = pair(w >> 16); r3 = pair(w >> 24);
+        const uint32_t w8 = w >> 8;
+        r0 = low(w); r1 = low(w8); r2 = high(w); r3 = high(w8);
+    }
+    __device__ static __forceinline__ uint32_t low(uint32_t w) {
+        const uint32_t v = (w & 0x000f000fu) | 0x64006400u, bias = 0xe408e408u;                               // -1032
+        const __half2 h = __hadd2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&bias));
+        return *reinterpret_cast<const uint32_t*>(&h);
+    }
+    __device__ static __forceinline__ uint32_t high(uint32_t w) {
+        const uint32_t v = (w & 0x00f000f0u) | 0x64006400u, unit = 0x2c002c00u, bias = 0xd480d480u;           // 1/16, -72
+        const __half2 h = __hfma2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&unit),
+                                  *reinterpret_cast<const __half2*>(&bias));
+        return *reinterpret_cast<const uint32_t*>(&h);
     }
 };
 
@@ -244,8 +268,9 @@ struct RowStream {
     // (g < ncols) load; the other columns multiply zeros.
     // Q4_K: unpacks the scales of the stage: lane l takes row l / 2, super-block l & 1, and leaves
     // per sub-block (d * scale, 1024 * d * scale + dmin * minimum): the codes enter the MMA as
-    // 1024 + q (a half built with two bit operations), and sum(x) of the sub-block takes both the
-    // 1024 and the minimum out again.
+    // 1024 + q (a half built with one bit operation), and sum(x) of the sub-block takes both the
+    // 1024 and the minimum out again. The odd sub-blocks are the high nibbles; they enter where they
+    // stand as 1024 + 16 q, with d * scale / 16 and 64 * d * scale + dmin * minimum.
     __device__ __forceinline__ void scales_k(uint32_t st, int nbc) {
         const int rr = lane >> 1, sb = lane & 1;
         if (sb * 8 < nbc) {
@@ -262,10 +287,11 @@ struct RowStream {
             float2* tab = reinterpret_cast<float2*>(const_cast<unsigned char*>(base) + stab + (uint32_t)rr * kKTablePitch + (uint32_t)sb * 64u);
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float s1 = __fmul_rn(d, (float)((scl >> (8 * j)) & 0xffu));
-                tab[j] = make_float2(s1, __fmaf_rn(1024.0f, s1, __fmul_rn(dmin, (float)((mnl >> (8 * j)) & 0xffu))));
-                const float t1 = __fmul_rn(d, (float)((sch >> (8 * j)) & 0xffu));
-                tab[4 + j] = make_float2(t1, __fmaf_rn(1024.0f, t1, __fmul_rn(dmin, (float)((mnh >> (8 * j)) & 0xffu))));
+                const float s1 = __fmul_rn(d, (float)((scl >> (8 * j)) & 0xffu)), m1 = __fmul_rn(dmin, (float)((mnl >> (8 * j)) & 0xffu));
+                const float s2 = __fmul_rn(d, (float)((sch >> (8 * j)) & 0xffu)), m2 = __fmul_rn(dmin, (float)((mnh >> (8 * j)) & 0xffu));
+                const float unit = j & 1 ? 0.0625f : 1.0f, off = j & 1 ? 64.0f : 1024.0f;      // odd sub-blocks: high nibbles
+                tab[j] = make_float2(__fmul_rn(s1, unit), __fmaf_rn(off, s1, m1));
+                tab[4 + j] = make_float2(__fmul_rn(s2, unit), __fmaf_rn(off, s2, m2));
             }
         }
     }
@@ -276,7 +302,8 @@ struct RowStream {
     __device__ __forceinline__ void chunk_k(uint32_t st, uint32_t xa, uint32_t xs, int nbc, float (&sum)[4]) {
         const uint32_t pA = st + (((uint32_t)g * kRowPitch + mA) & ~3u), sA = (mA & 3u) * 8u;
         const uint32_t pB = st + (((uint32_t)(8 + g) * kRowPitch + mB) & ~3u), sB = (mB & 3u) * 8u;
-        auto nib = [](uint32_t w, int shift) { return ((w >> shift) & 0x000f000fu) | 0x64006400u; };   // two halves 1024 + q
+        auto low = [](uint32_t w) { return (w & 0x000f000fu) | 0x64006400u; };    // two halves 1024 + q
+        auto high = [](uint32_t w) { return (w & 0x00f000f0u) | 0x64006400u; };   // two halves 1024 + 16 q
 #pragma unroll
         for (int sb = 0; sb < 2; sb++) {
             if (FULL || sb * 8 < nbc) {
@@ -297,10 +324,11 @@ struct RowStream {
                     const float4 tb = *reinterpret_cast<const float4*>(base + stab + (uint32_t)(8 + g) * kKTablePitch + kb * 8);
                     const float4 xv = *reinterpret_cast<const float4*>(base + xs + kb * 8);   // (hi, lo) sums of kb and kb + 1
                     float lo[4], hi[4];
-                    mma16816_first(lo, nib(wa0, 0), nib(wb0, 0), nib(wa0, 8), nib(wb0, 8), xl.x, xl.y);
-                    mma16816(lo, nib(wa1, 0), nib(wb1, 0), nib(wa1, 8), nib(wb1, 8), xl.z, xl.w);
-                    mma16816_first(hi, nib(wa0, 4), nib(wb0, 4), nib(wa0, 12), nib(wb0, 12), xh.x, xh.y);
-                    mma16816(hi, nib(wa1, 4), nib(wb1, 4), nib(wa1, 12), nib(wb1, 12), xh.z, xh.w);
+                    const uint32_t va0 = wa0 >> 8, va1 = wa1 >> 8, vb0 = wb0 >> 8, vb1 = wb1 >> 8;
+                    mma16816_first(lo, low(wa0), low(wb0), low(va0), low(vb0), xl.x, xl.y);
+                    mma16816(lo, low(wa1), low(wb1), low(va1), low(vb1), xl.z, xl.w);
+                    mma16816_first(hi, high(wa0), high(wb0), high(va0), high(vb0), xh.x, xh.y);
+                    mma16816(hi, high(wa1), high(wb1), high(va1), high(vb1), xh.z, xh.w);
                     sum[0] = __fmaf_rn(lo[0], ta.x, __fmaf_rn(-ta.y, xv.x, sum[0]));
                     sum[1] = __fmaf_rn(lo[1], ta.x, __fmaf_rn(-ta.y, xv.y, sum[1]));
                     sum[2] = __fmaf_rn(lo[2], tb.x, __fmaf_rn(-tb.y, xv.x, sum[2]));
@@ -451,19 +479,15 @@ __host__ __device__ inline size_t token_smem_bytes(int fmt, int nkb, int stages)
 }
 
 // Splits f32 values into hi + lo halves and scatters them into the B-fragment layout:
-// frag[((kb * 2 + col) * 4 + tig) * 4 + slot] is a half2 (element 4*tig+slot, element 4*tig+slot+16)
-// of block kb; hi goes to column 0, lo to column 1.
-// Q4_K delivers elements 8*tig .. 8*tig+7 of a sub-block to lane tig: slots 0, 1 hold (e0, e2), (e1, e3),
-// slots 2, 3 the same of e4..e7.
+// frag[((kb * 2 + col) * 4 + tig) * 4 + slot] is a half2 of two elements of block kb (frag_place); hi goes to
+// column 0, lo to column 1.
 __device__ __forceinline__ void frag_store(__half* frag, int k, float v, int fmt) {
     __half hi = __float2half_rn(v);
     float rem = nonfinite(v) ? 0.0f : v - __half2float(hi);
     __half lo = __float2half_rn(rem);
-    int kb = k >> 5, j = k & 31, jj = j & 15, sel = j >> 4, tig = jj >> 2, slot = jj & 3;
-    if (fmt == OCO_FMT_Q4_K) {
-        const int r = j & 7;
-        tig = j >> 3; slot = (r >> 2) * 2 + (r & 1); sel = (r >> 1) & 1;
-    }
+    int tig, slot, sel;
+    frag_place(fmt, k & 31, tig, slot, sel);
+    const int kb = k >> 5;
     size_t at = ((((size_t)kb * 2) * 4 + tig) * 4 + slot) * 2 + sel;
     frag[at] = hi;
     frag[at + (size_t)16 * 2] = lo;  // next column: 4 tig * 4 slots * 2 halves further

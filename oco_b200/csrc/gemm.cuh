@@ -189,17 +189,18 @@ __device__ __forceinline__ void decode_q4_0_block(const uint32_t* w, uint32_t sh
         q[0] = __funnelshift_rc(w[1], w[2], s3); q[1] = __funnelshift_rc(w[2], w[3], s3);
         q[2] = __funnelshift_rc(w[3], w[4], s3); q[3] = __funnelshift_rc(w[4], w[5], s3);
     }
-    const uint32_t bias = 0x64086408u;  // 1032 as halves: (1024 + q) - 1032 = q - 8
+    // A code byte is copied under 0x64 in both halves; one mask leaves the low nibble as 1024 + q and the high
+    // one, where it stands, as 1024 + 16 q; one exact fused multiply-add makes q - 8 of both.
+    const uint32_t unit = 0x2c003c00u, bias = 0xd480e408u;              // (1, 1/16), (-1032, -72)
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint32_t lo = q[i] & 0x0f0f0f0fu, hi = (q[i] >> 4) & 0x0f0f0f0fu;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            // byte j of lo -> bits 0..7, byte j of hi -> bits 16..23, 0x64 above each: halves 1024 + q
-            uint32_t v = (__byte_perm(lo, hi, (uint32_t)(j | ((4 + j) << 8))) & 0x00ff00ffu) | 0x64006400u;
-            __half2 h = __hsub2(*reinterpret_cast<__half2*>(&v), *reinterpret_cast<const __half2*>(&bias));
-            __half2 o = __hmul2(h, *reinterpret_cast<const __half2*>(&d2));
-            out[4 * i + j] = *reinterpret_cast<uint32_t*>(&o);
+            const uint32_t v = __byte_perm(q[i], 0x64646464u, 0x4040u | (uint32_t)(j | (j << 8))) & 0xfff0ff0fu;
+            const __half2 h = __hfma2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&unit),
+                                      *reinterpret_cast<const __half2*>(&bias));
+            const __half2 o = __hmul2(h, *reinterpret_cast<const __half2*>(&d2));
+            out[4 * i + j] = *reinterpret_cast<const uint32_t*>(&o);
         }
     }
 }
