@@ -197,6 +197,7 @@ struct RowStream {
     const uint8_t* spanB;      // both advanced to the first block of the range
     uint32_t row_bytes, total_bytes;
     int nchunks, nb, kb_first;
+    bool ahead = false;        // the unit's first stage was started under the unit before (run's `next`)
     // per lane
     uint32_t mK = 0;           // Q4_K: misalignment of row lane / 2 (the row whose scales this lane unpacks)
     uint32_t xsum = 0;         // Q4_K: byte offset in shared memory of the fragments' per-block sums
@@ -239,7 +240,9 @@ struct RowStream {
             alB[c] = qb & ~3u; shB[c] = (qb & 3u) * 8u;
         }
 #pragma unroll
-        for (int s = 0; s < STAGES - 1; s++) issue(s);
+        for (int s = 0; s < STAGES - 1; s++)
+            if (s > 0 || !ahead) issue(s);
+        ahead = false;
     }
 
     // Starts the copies of chunk c of the unit (nothing past the last chunk). The stage was read
@@ -247,12 +250,14 @@ struct RowStream {
     __device__ __forceinline__ void issue(int c) {
         if (c >= nchunks) return;
         const uint32_t off = (uint32_t)c * kChunkBytes;
-        const uint32_t len = min(kChunkBytes, total_bytes - off);
-        const uint32_t stage = (seq + (uint32_t)c) % STAGES;
+        copy_rows((lane < 8 ? spanA : spanB) + (size_t)(lane & 7) * row_bytes, off, min(kChunkBytes, total_bytes - off), (uint32_t)c);
+    }
+
+    // Lanes 0..15 copy one row each into the stage of chunk c; the byte total of the stage is summed over them first.
+    __device__ __forceinline__ void copy_rows(const uint8_t* row, uint32_t off, uint32_t len, uint32_t c) {
+        const uint32_t stage = (seq + c) % STAGES;
         const uint32_t bar = bars + 8u * stage;
         const uint32_t dst = base_addr + ring + stage * kStageBytes;
-        // lanes 0..15 copy one row each; the byte total of the stage is summed over them first
-        const uint8_t* row = (lane < 8 ? spanA : spanB) + (size_t)(lane & 7) * row_bytes;
         const uint32_t m = (uint32_t)(uintptr_t)row & 15u;
         const uint32_t bytes = lane < 16 ? ((m + len + 15u) & ~15u) : 0u;
         uint32_t total = bytes;
@@ -392,10 +397,19 @@ struct RowStream {
         }
     }
 
-    // xaddr: byte offset in shared memory of this lane's B fragment (uint4) for block kb0.
-    __device__ __forceinline__ void run(uint32_t xaddr, float (&sum)[4]) {
+    // xaddr: byte offset in shared memory of this lane's B fragment (uint4) for block kb0. nextA, nextB: the spans
+    // of the warp's next unit (same row length and block range), whose first stage then travels under this unit's
+    // last one; null: there is none, or begin() starts it.
+    __device__ __forceinline__ void run(uint32_t xaddr, float (&sum)[4], const uint8_t* nextA = nullptr, const uint8_t* nextB = nullptr) {
+        static_assert(STAGES == 2, "the next unit's first stage takes the place of the stage past the last one");
         for (int c = 0; c < nchunks; c++) {
-            issue(c + STAGES - 1);
+            if (c + 1 < nchunks) {
+                issue(c + 1);
+            } else if (nextA) {
+                copy_rows((lane < 8 ? nextA : nextB) + (size_t)kb_first * B::kBytes + (size_t)(lane & 7) * row_bytes, 0u,
+                          min(kChunkBytes, total_bytes), (uint32_t)nchunks);
+                ahead = true;
+            }
             const uint32_t n = seq + (uint32_t)c, stage = n % STAGES;
             mbar_wait(bars + 8u * stage, (n / STAGES) & 1u, abort_flag, status);
             const uint32_t st = ring + stage * kStageBytes;
