@@ -536,6 +536,12 @@ struct DecodeExpandParams {
     uint32_t row_bytes;      // bytes from one gate (or up) row to the next: the packed length of a row of H
                              // elements, or twice that when gate and up rows are interleaved in one tensor
     int bias_stride;         // floats from one feature's bias to the next (1, or 2 when interleaved)
+    // The always-on expert (not gated; sh_F 0: none): its units follow the routed ones in the same launch.
+    const uint8_t* sh_up_w;
+    float* sh_act;
+    __half* sh_actfrag;
+    int sh_F;
+    uint32_t sh_row_bytes;
     uint32_t* status;        // device status word: a copy that never arrives is reported here
 };
 
@@ -563,7 +569,8 @@ __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_expand_kernel(c
     const int ksplit = p.ksplit, group = warp / ksplit, s = warp - group * ksplit;
     const int groups = WARPS / ksplit;
     const int col_blocks = p.F / COLS;
-    const int units = p.K * col_blocks;
+    const int routed = p.K * col_blocks;
+    const int units = routed + (GATED ? 0 : p.sh_F / COLS);
     const int nslots = gridDim.x * groups;
     int bps = (nkb + ksplit - 1) / ksplit;
     if (FMT == OCO_FMT_Q4_K) bps = (bps + 7) & ~7;          // whole super-blocks
@@ -583,11 +590,17 @@ __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_expand_kernel(c
     }
     bool fetched = false;
     for (int unit = blockIdx.x * groups + group; unit < units; unit += nslots) {
-        const int r = unit / col_blocks, c0 = (unit - r * col_blocks) * COLS;
-        const uint32_t e = __shfl_sync(0xffffffffu, p.ids ? __ldg(p.ids + r) : 0u, 0);
-        const size_t off = ((size_t)e * p.F + c0) * p.row_bytes;
-        if (GATED) rs.begin(p.gate_w + off, p.up_w + off, p.row_bytes, kb0, nb);
-        else rs.begin(p.up_w + off, p.up_w + off + (size_t)8 * p.row_bytes, p.row_bytes, kb0, nb);
+        const bool sh = !GATED && unit >= routed;
+        const int r = sh ? 0 : unit / col_blocks, c0 = (unit - (sh ? routed : r * col_blocks)) * COLS;
+        const uint32_t e = __shfl_sync(0xffffffffu, p.ids && !sh ? __ldg(p.ids + r) : 0u, 0);
+        const uint32_t rb = sh ? p.sh_row_bytes : p.row_bytes;
+        const size_t off = ((size_t)e * p.F + c0) * rb;
+        if (GATED) {
+            rs.begin(p.gate_w + off, p.up_w + off, rb, kb0, nb);
+        } else {
+            const uint8_t* span = (sh ? p.sh_up_w : p.up_w) + off;
+            rs.begin(span, span + (size_t)8 * rb, rb, kb0, nb);
+        }
         float b0 = 0.f, b1 = 0.f;
         if (ARCH == OCO_ARCH_GPT_OSS && s == 0 && tig == 0) {   // biases travel while the rows stream
             b0 = __ldg(p.gate_b + ((size_t)e * p.F + c0 + g) * p.bias_stride);
@@ -600,8 +613,8 @@ __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_expand_kernel(c
         join_split(part, warp, group, s, ksplit, g, tig, r0, r1);
         if (s == 0 && tig == 0) {
             auto put = [&](int col, float v) {
-                p.act[(size_t)r * p.F + col] = v;
-                frag_store(p.actfrag + (size_t)r * (p.F / 32) * (kFragBlockBytes / 2), col, v, FMT);
+                (sh ? p.sh_act : p.act + (size_t)r * p.F)[col] = v;
+                frag_store(sh ? p.sh_actfrag : p.actfrag + (size_t)r * (p.F / 32) * (kFragBlockBytes / 2), col, v, FMT);
             };
             if (ARCH == OCO_ARCH_GPT_OSS) {
                 float gate = __fadd_rn(r0, bf16_round(b0));
@@ -634,8 +647,16 @@ struct DecodeDownParams {
     uint32_t* arrivals;       // one zeroed counter per block of 16 output rows; left at zero again
     const float* probs;       // [K]
     uint16_t* residual;       // bf16 [H], in place
-    const uint16_t* shared;   // bf16 [H] shared-expert output joining the sum, or null
     int round_sum;            // 1: the expert sum is rounded to bf16 before the residual add
+    // The always-on expert (sh_F 0: none), one more route of its own width in the same launch: its output joins the
+    // sum ahead of the routed ones, its row blocks count as one arrival more.
+    const uint8_t* sh_down_w;
+    const __half* sh_actfrag; // [sh_F / 32] blocks of 128 bytes
+    uint16_t* shared;         // bf16 [H], written here, joined by the combine
+    int sh_F;
+    uint32_t sh_row_bytes;
+    int sh_shares;            // CTAs go round K + sh_shares places: one for each route, sh_shares for the always-on expert
+    int sh_ksplit;            // warps per unit of the always-on expert
     uint32_t* status;         // device status word
 };
 
@@ -648,9 +669,15 @@ __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_down_kernel(con
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int nkb = p.F / 32;
-    const int route = blockIdx.x % p.K, idx = blockIdx.x / p.K, ctas = gridDim.x / p.K;
-    if (idx >= ctas) return;
+    // the CTA's place: a route, or (with sh_shares places, the work of a route being one) the always-on expert
+    const int places = p.K + p.sh_shares, place = blockIdx.x % places, turn = blockIdx.x / places, turns = gridDim.x / places;
+    if (turn >= turns) return;
+    const bool sh = place >= p.K;
+    const int route = sh ? 0 : place;
+    const int idx = sh ? turn * p.sh_shares + place - p.K : turn, ctas = sh ? turns * p.sh_shares : turns;
+    const int nkb = (sh ? p.sh_F : p.F) / 32;
+    const uint32_t row_bytes = sh ? p.sh_row_bytes : p.row_bytes;
+    uint16_t* y = sh ? p.shared : p.y + (size_t)route * p.H;
     const uint32_t part_off = frag_region_bytes(FMT, nkb);
     float* part = reinterpret_cast<float*>(smem + part_off);
     volatile uint32_t* give_up = reinterpret_cast<volatile uint32_t*>(part) + 496;
@@ -660,7 +687,7 @@ __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_down_kernel(con
     pdl_launch_dependents();
     if (tid == 0) *give_up = 0u;
 
-    const int ksplit = p.ksplit, group = warp / ksplit, s = warp - group * ksplit;
+    const int ksplit = sh ? p.sh_ksplit : p.ksplit, group = warp / ksplit, s = warp - group * ksplit;
     const int groups = WARPS / ksplit;
     const int row_blocks = p.H / 16;
     const int nslots = ctas * groups;
@@ -674,8 +701,8 @@ __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_down_kernel(con
     rs.xsum = (uint32_t)nkb * kFragBlockBytes;
     pdl_wait();               // the expand kernel's fragments are complete
     // the route's activation fragments (written by the expand kernel)
-    fetch_fragments(smem, p.actfrag + (size_t)route * nkb * (kFragBlockBytes / 2), (uint32_t)nkb * kFragBlockBytes, xbar, warp, lane);
-    const uint32_t e = __shfl_sync(0xffffffffu, p.ids ? __ldg(p.ids + route) : 0u, 0);
+    fetch_fragments(smem, sh ? p.sh_actfrag : p.actfrag + (size_t)route * nkb * (kFragBlockBytes / 2), (uint32_t)nkb * kFragBlockBytes, xbar, warp, lane);
+    const uint32_t e = __shfl_sync(0xffffffffu, p.ids && !sh ? __ldg(p.ids + route) : 0u, 0);
     __syncthreads();          // the mbarriers exist
     if (FMT == OCO_FMT_Q4_K) {
         mbar_wait(xbar, 0u, give_up, p.status);
@@ -685,8 +712,8 @@ __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_down_kernel(con
     bool fetched = false;
     for (int rb = idx * groups + group; rb < row_blocks; rb += nslots) {
         const int d0 = rb * 16;
-        const uint8_t* span = p.down_w + ((size_t)e * p.H + d0) * p.row_bytes;
-        rs.begin(span, span + (size_t)8 * p.row_bytes, p.row_bytes, kb0, nb);
+        const uint8_t* span = (sh ? p.sh_down_w : p.down_w) + ((size_t)e * p.H + d0) * row_bytes;
+        rs.begin(span, span + (size_t)8 * row_bytes, row_bytes, kb0, nb);
         float b0 = 0.f, b1 = 0.f;
         if (p.down_b && s == 0 && tig == 0) {
             b0 = __ldg(p.down_b + (size_t)e * p.H + d0 + g);
@@ -700,24 +727,25 @@ __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_down_kernel(con
         if (s != 0) continue;
         if (tig == 0) {
             if (p.down_b) { r0 = __fadd_rn(r0, bf16_round(b0)); r1 = __fadd_rn(r1, bf16_round(b1)); }
-            p.y[(size_t)route * p.H + d0 + g] = f32_to_bf16_bits(r0);
-            p.y[(size_t)route * p.H + d0 + 8 + g] = f32_to_bf16_bits(r1);
+            y[d0 + g] = f32_to_bf16_bits(r0);
+            y[d0 + 8 + g] = f32_to_bf16_bits(r1);
         }
         if (p.residual) {
             // Whoever finishes a row block last combines it. No warp waits for another.
             __threadfence();
             __syncwarp();
+            const uint32_t last = (uint32_t)(p.K - 1 + (p.sh_F ? 1 : 0));
             uint32_t seen = 0;
             if (lane == 0) {
                 seen = atomicAdd(p.arrivals + rb, 1u);
-                if (seen == (uint32_t)(p.K - 1)) p.arrivals[rb] = 0;   // ready for the next call on this stream
+                if (seen == last) p.arrivals[rb] = 0;   // ready for the next call on this stream
             }
             seen = __shfl_sync(0xffffffffu, seen, 0);
             // (a step during which a bounded wait gave up leaves the residual as it was)
-            if (seen == (uint32_t)(p.K - 1) && lane < 16 && *reinterpret_cast<volatile uint32_t*>(p.status) == 0u) {
+            if (seen == last && lane < 16 && *reinterpret_cast<volatile uint32_t*>(p.status) == 0u) {
                 __threadfence();
                 const int row = d0 + lane;
-                float sres = p.shared ? bf16_bits_to_f32(p.shared[row]) : 0.0f;
+                float sres = p.sh_F ? bf16_bits_to_f32(__ldcg(p.shared + row)) : 0.0f;
                 for (int r = 0; r < p.K; r++)
                     sres = __fmaf_rn(bf16_bits_to_f32(__ldcg(p.y + (size_t)r * p.H + row)), p.probs[r], sres);
                 if (p.round_sum) sres = bf16_round(sres);
