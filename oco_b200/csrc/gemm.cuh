@@ -205,33 +205,6 @@ __device__ __forceinline__ void decode_q4_0_block(const uint32_t* w, uint32_t sh
     }
 }
 
-// Two f32 values in one register pair; the packed operations round each of them as the scalar ones do.
-__device__ __forceinline__ uint64_t f32x2(float a, float b) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t f32x2_bits(uint32_t a, uint32_t b) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // Q4_K: code bytes 16h..16h+15 of sub-blocks 2c and 2c+1 of one super-block -> 16 half2 in operand
 // order: each byte gives half2( d*sc0*q_lo - dmin*m0 , d*sc1*q_hi - dmin*m1 ), with one f32 rounding
 // in the subtraction before the half rounding (weights.metal:67-77).
@@ -265,7 +238,7 @@ __device__ __forceinline__ void decode_q4_k_half(const uint32_t* hdr, const uint
             const uint64_t q = add_f32x2(f32x2_bits((word & (0x0fu << at)) | kMagic, (word & (0xf0u << at)) | kMagic), unmagic);
             const uint64_t v = fma_f32x2(q, (j & 1) ? scale8 : scale0, minus_min);
             float lo, hi;
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+            f32x2_split(v, lo, hi);
             const __half2 o = __floats2half2_rn(lo, hi);
             out[4 * i + j] = *reinterpret_cast<const uint32_t*>(&o);
         }
