@@ -486,6 +486,32 @@ def test_nemotron_few_tokens_streamed(moe, oracle, tokens):
     check_layer(moe, oracle, layer, tokens, seed=tokens)
 
 
+@pytest.mark.parametrize("arch,hidden,ffn,experts,top_k,tokens",
+                         [("gpt_oss", 96, 96, 32, 4, 3), ("gpt_oss", 288, 320, 32, 4, 64), ("gpt_oss", 640, 160, 128, 4, 250),
+                          ("nemotron", 256, 160, 128, 6, 90), ("nemotron", 96, 1056, 16, 2, 2), ("qwen", 256, 256, 16, 4, 2),
+                          ("qwen", 512, 768, 128, 8, 9), ("qwen", 768, 512, 128, 8, 100)])
+def test_few_tokens_equal_shares(moe, oracle, arch, hidden, ffn, experts, top_k, tokens):
+    """The persistent few-token kernel: fewer units than warps, a last round that some warps have no unit in, CTAs whose
+    run of rounds ends inside a group or spans several, fewer rounds than CTAs."""
+    if arch == "gpt_oss":
+        layer = synth.make_layer(synth.ARCH_GPT_OSS, hidden, ffn, experts, top_k, synth.FMT_MXFP4, seed=hidden + ffn)
+    elif arch == "qwen":
+        layer = synth.make_layer(synth.ARCH_QWEN, hidden, ffn, experts, top_k, synth.FMT_Q4_K, seed=hidden + ffn)
+    else:
+        layer = synth.make_layer(synth.ARCH_NEMOTRON, hidden, ffn, experts, top_k, synth.FMT_Q4_0, seed=hidden + ffn, shared_ffn=64,
+                                 normalize=True, scale=2.5)
+    check_layer(moe, oracle, layer, tokens, seed=tokens, residual="normal")
+    check_layer(moe, oracle, layer, tokens, seed=tokens + 1, misalign=5)
+
+
+@pytest.mark.parametrize("ffn,shared_ffn,top_k", [(192, 64, 6), (160, 1920, 2), (96, 96, 6), (64, 4096, 1)])
+def test_nemotron_single_token_always_on_expert(moe, oracle, ffn, shared_ffn, top_k):
+    """The always-on expert in the routed launches: narrower than, as wide as and much wider than a routed one."""
+    layer = synth.make_layer(synth.ARCH_NEMOTRON, 352, ffn, 16, top_k, synth.FMT_Q4_0, seed=ffn, shared_ffn=shared_ffn, normalize=True, scale=2.5)
+    check_layer(moe, oracle, layer, 1, seed=ffn, residual="normal")
+    check_layer(moe, oracle, layer, 1, seed=ffn + 1, misalign=7)
+
+
 @pytest.mark.parametrize("tokens", [1, 3])
 def test_wide_layer_falls_back_to_tiles(moe, oracle, tokens):
     """hidden = 8192 is too wide for the token's fragments to share the SM with the streaming rings:
