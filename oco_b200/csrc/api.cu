@@ -788,11 +788,11 @@ int stage_experts(oco_moe_plan* plan, const uint16_t* x, const uint32_t* ids, in
     Workspace& ws = plan->ws;
     const int H = d.hidden, F = d.ffn, E = d.experts;
     const int live = rs.expected > 0 && rs.expected < R ? rs.expected : R;   // routes expected to carry this plan's experts
-    if (FMT != OCO_FMT_Q4_K && d.numerics == 0 && live <= plan->batch_max_avg * E && (rs.expected == 0 || R <= 64 * E) && !plan->no_batch_path &&
-        batch_smem_bytes(H / 32) <= kMaxDynamicSmem && batch_smem_bytes(F / 32) <= kMaxDynamicSmem) {
+    if (d.numerics == 0 && live <= plan->batch_max_avg * E && (rs.expected == 0 || R <= 64 * E) && !plan->no_batch_path &&
+        batch_smem_bytes(FMT, H / 32) <= kMaxDynamicSmem && batch_smem_bytes(FMT, F / 32) <= kMaxDynamicSmem) {
         // A few routes per expert: memory-bound, streamed with up to eight routes per MMA (batch.cuh).
         // (Layers too wide for the fragments to sit in shared memory take the tiles.)
-        if constexpr (FMT != OCO_FMT_Q4_K) {
+        {
             plan->last_tile_rows = kBatchCols;
             launch_route_plan(plan, ids, R, E, kBatchCols, rs, st);
             const int groups = (int)batch_max_groups((size_t)R, (size_t)E);
@@ -817,13 +817,13 @@ int stage_experts(oco_moe_plan* plan, const uint16_t* x, const uint32_t* ids, in
             bp.frag_in = ws.bfrag_in; bp.frag_out = ws.bfrag_out; bp.out = ws.act;
             bp.n_in = H; bp.n_out = F; bp.row_bytes = plan->up_row_stride; bp.bias_stride = plan->up_bias_stride;
             mark(plan, st, "up_rows");
-            CK(launch_dependent(batch_rows_kernel<FMT, EPI_UP>, up_grid, dim3(kBatchThreads), batch_smem_bytes(H / 32), st, bp));
+            CK(launch_dependent(batch_rows_kernel<FMT, EPI_UP>, up_grid, dim3(kBatchThreads), batch_smem_bytes(FMT, H / 32), st, bp));
             bp.w0 = plan->w.down_w; bp.w1 = nullptr;
             bp.b0 = ARCH == OCO_ARCH_GPT_OSS ? plan->w.down_b : nullptr; bp.b1 = nullptr;
             bp.frag_in = ws.bfrag_out; bp.frag_out = nullptr; bp.out = y;
             bp.n_in = F; bp.n_out = H; bp.row_bytes = plan->down_row_bytes; bp.bias_stride = 1;
             mark(plan, st, "down_rows");
-            CK(launch_dependent(batch_rows_kernel<FMT, kEpiDownBf16>, down_grid, dim3(kBatchThreads), batch_smem_bytes(F / 32), st, bp));
+            CK(launch_dependent(batch_rows_kernel<FMT, kEpiDownBf16>, down_grid, dim3(kBatchThreads), batch_smem_bytes(FMT, F / 32), st, bp));
             plan->launches += 2;
             CK(cudaGetLastError());
             return OCO_OK;
@@ -1036,6 +1036,10 @@ int oco_moe_plan_create(const oco_moe_desc* desc, oco_moe_plan** out) {
     { const char* e = getenv("OCO_MOE_TOKEN_MX"); plan->mx_on = e && e[0] == '1'; }
     { const char* e = getenv("OCO_MOE_ROUTE_PLAN_SINGLE_MAX"); if (e && atoi(e) >= 0) plan->route_plan_single_max = atoi(e); }
     { const char* e = getenv("OCO_MOE_REPACKED_TOKEN"); plan->rp_token_on = e && e[0] == '1'; }
+    // Q4_K decodes twice the instructions per weight of the other formats on the streamed path (half weights from a scale
+    // and a minimum): the tiles draw level earlier. Qwen3 layer, streamed | tiles: 96 rows (6 routes per expert) 250 |
+    // 305 us, 128 rows (8) 312 | 307.
+    if (d.weight_format == OCO_FMT_Q4_K) plan->batch_max_avg = 6;
     { const char* e = getenv("OCO_MOE_BATCH_MAX_AVG"); if (e && atoi(e) > 0) plan->batch_max_avg = atoi(e) < 64 ? atoi(e) : 64; }
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) == cudaSuccess &&

@@ -21,15 +21,20 @@ constexpr int kBatchThreads = kBatchWarps * 32;
 constexpr int kBatchCols = 8;
 constexpr int kBatchFragBlock = kBatchCols * 64;    // bytes of one block's B fragments
 
-__host__ __device__ inline size_t batch_smem_bytes(int nkb) {
-    return (size_t)nkb * kBatchFragBlock + kMiscBytes + (size_t)kBatchWarps * kScaleBytes +
+__host__ __device__ inline size_t batch_smem_bytes(int fmt, int nkb) {
+    return (size_t)nkb * kBatchFragBlock + kMiscBytes + (size_t)kBatchWarps * scale_table_bytes(fmt) +
            (size_t)kBatchWarps * 2 * kStageBytes + 16;
 }
 
-// Position (in halves) of element k of column `col` in a group's fragments (frag_place within the block).
+// Position (in halves) of element k of column `col` in a group's fragments: frag_place within the block, but for Q4_K
+// neighbours (RowStream::chunk_kh).
 __host__ __device__ inline size_t batch_frag_pos(int fmt, int k, int col) {
     int tig, slot, sel;
-    frag_place(fmt, k & 31, tig, slot, sel);
+    if (fmt == OCO_FMT_Q4_K) {
+        tig = (k & 31) >> 3; slot = (k & 7) >> 1; sel = k & 1;
+    } else {
+        frag_place(fmt, k & 31, tig, slot, sel);
+    }
     return ((((size_t)(k >> 5) * kBatchCols + col) * 4 + tig) * 4 + slot) * 2 + sel;
 }
 
@@ -55,13 +60,19 @@ __global__ void __launch_bounds__(256) batch_fragments_kernel(const uint16_t* __
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (col < n) {
             const uint32_t token = route_of_row[row0 + col] / (uint32_t)per_row;
-            const uint16_t* src = x + (size_t)token * H + kb * 32 + 4 * tig;
-            const uint2 lo = *reinterpret_cast<const uint2*>(src), hi = *reinterpret_cast<const uint2*>(src + 16);
+            // elements 4 tig .. 4 tig + 3 and the same of the elements 16 further; Q4_K: 8 tig .. 8 tig + 7
+            const uint16_t* src = x + (size_t)token * H + kb * 32 + (FMT == OCO_FMT_Q4_K ? 8 : 4) * tig;
+            const uint2 lo = *reinterpret_cast<const uint2*>(src), hi = *reinterpret_cast<const uint2*>(src + (FMT == OCO_FMT_Q4_K ? 4 : 16));
             auto pair = [](uint32_t a, uint32_t b) {          // (bf16 a, bf16 b) -> half2
                 __half2 h = __floats2half2_rn(__uint_as_float(a << 16), __uint_as_float(b << 16));
                 return *reinterpret_cast<uint32_t*>(&h);
             };
-            if (FMT == OCO_FMT_Q4_0) {                        // elements two apart (frag_place)
+            if (FMT == OCO_FMT_Q4_K) {                        // neighbours (batch_frag_pos)
+                v.x = pair(lo.x & 0xffffu, lo.x >> 16);
+                v.y = pair(lo.y & 0xffffu, lo.y >> 16);
+                v.z = pair(hi.x & 0xffffu, hi.x >> 16);
+                v.w = pair(hi.y & 0xffffu, hi.y >> 16);
+            } else if (FMT == OCO_FMT_Q4_0) {                 // elements two apart (frag_place)
                 v.x = pair(lo.x & 0xffffu, lo.y & 0xffffu);
                 v.y = pair(lo.x >> 16, lo.y >> 16);
                 v.z = pair(hi.x & 0xffffu, hi.y & 0xffffu);
@@ -100,7 +111,8 @@ struct BatchParams {
 // (or fewer) the last wave decided: 19 groups made 152 CTAs of three rounds on 148 SMs, six rounds where three
 // suffice. Within its run a warp starts the next unit's first stage under the last stage of the one before, across
 // groups too, so that its rows never stop; only the group's fragments are waited for when the group changes.
-// gpt-oss-20b-shaped step of 7 tokens 177 -> 137 us, 120b-shaped one of 64 tokens 517 -> 494 us.
+// gpt-oss-20b-shaped step of 7 tokens 177 -> 137 us, 120b-shaped one of 64 tokens 517 -> 494 us. Qwen3 (Q4_K), which
+// took 256-route tiles for any batch: 2 rows 136 -> 66 us, 8 rows 352 -> 130, 32 rows 254 -> 200, 96 rows 306 -> 250.
 template <int FMT, int EPI>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_rows_kernel(const BatchParams p) {
     constexpr bool GATED = epi_gated(EPI);
@@ -114,8 +126,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_rows_kernel(const Batc
     float* misc = reinterpret_cast<float*>(smem + part_off);
     volatile uint32_t* give_up = reinterpret_cast<volatile uint32_t*>(misc) + 496;
     const uint32_t xbar = smem_u32(smem) + part_off + 1920u;
-    const uint32_t stab = part_off + kMiscBytes + (uint32_t)warp * kScaleBytes;
-    const uint32_t ring = part_off + kMiscBytes + (uint32_t)kBatchWarps * kScaleBytes + (uint32_t)warp * 2 * kStageBytes;
+    const uint32_t stab = part_off + kMiscBytes + (uint32_t)warp * scale_table_bytes(FMT);
+    const uint32_t ring = part_off + kMiscBytes + (uint32_t)kBatchWarps * scale_table_bytes(FMT) + (uint32_t)warp * 2 * kStageBytes;
     pdl_launch_dependents();
     RowStream<FMT, 2, kBatchCols> rs;
     rs.init(smem, ring, stab, part_off + 1280u + (uint32_t)warp * 16u, give_up, p.status, lane);
