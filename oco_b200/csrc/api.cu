@@ -2,6 +2,7 @@
 // The sequencing mirrors the reference operators it replaces:
 //   Bindings::experts        src/weights/compute/feed_forward.rs:107-275
 //   Bindings::relu_experts   src/weights/compute/nemotron.rs:286-545
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -48,6 +49,7 @@ struct Workspace {
     float* act1 = nullptr;        // f32 [K, F] single-token activations
     __half* actfrag = nullptr;    // single-token B fragments of the down projection
     __half* xfrag = nullptr;      // single-token B fragments of the token itself
+    float* split_partial = nullptr;  // f32 partial sums of a split dense product
     __half* bfrag_in = nullptr;   // few-token path: B fragments of each route group, input rows
     __half* bfrag_out = nullptr;  //                 and activations
     uint32_t* arrivals = nullptr; // single-token combine: one counter per output row (or row block), then the router's
@@ -193,6 +195,9 @@ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Lays the workspace out; with base == nullptr only the total is meaningful.
 // Route groups (up to eight routes of one expert) that R routes over E experts can form.
+// CTAs that a split dense product may use, whatever the GPU has: bounds its partial sums in the workspace.
+constexpr int kSplitCtas = 148;
+
 size_t batch_max_groups(size_t R, size_t E) { return R / 8 + (E < R ? E : R); }
 
 Workspace carve(const oco_moe_desc& d, int max_rows, unsigned char* base) {
@@ -236,6 +241,15 @@ Workspace carve(const oco_moe_desc& d, int max_rows, unsigned char* base) {
         w.sh_act1 = (float*)take(S * 4);
         w.sh_actfrag = (__half*)take((S / 32) * 128 * 2);
         w.sh_ids = (uint32_t*)take(256);
+    }
+    if (S || (E == 1 && d.numerics == 0)) {
+        // partial sums of a split dense product: at most kSplitCtas items of 256 x 256 outputs
+        auto parts = [&](size_t n) {
+            const size_t most = (size_t)kSplitCtas / ((n + 255) / 256);
+            return most < 2 ? (size_t)0 : std::min((size_t)kSplitCtas * 256 * 256, most * T * n);
+        };
+        const size_t floats = std::max(parts(H), parts(F));
+        if (floats) w.split_partial = (float*)take(floats * 4);
     }
     w.norm = (uint16_t*)take(T * H * 2);
     if (d.weight_format == OCO_FMT_MXFP4) {
@@ -394,6 +408,36 @@ int launch_gemm_wide(oco_moe_plan* plan, GemmParams gp, const CUtensorMap* maps,
         plan->launches++;
         CK(cudaGetLastError());
         return OCO_OK;
+    }
+    if constexpr (EPI == kEpiDownBf16) {
+        // A dense product of a few hundred rows has fewer items than the GPU has SMs, and each walks the whole
+        // contraction: 512 rows of a 6144 -> 2048 product are 16 items of 96 slices. The contraction is then split, an
+        // item per part, and the f32 parts are added in order. A slice takes about a microsecond; writing and reading
+        // a part costs its eight bytes per output at about 4 TB/s, and the second launch about four microseconds.
+        // Whole | split: 2048 -> 6144 -> 2048 (Q4_K) 16 rows 124 | 51 us, 512 rows 155 | 82, 1500 rows 203 | 155; 2880 x 2880
+        // (MXFP4) 16 rows 35 | 16, 512 rows 45 | 30, 1500 rows 53 | 52; Nemotron-H layer of 1000 tokens 627 | 605.
+        if (!gp.tiles && !gp.b0 && plan->ws.split_partial) {
+            const int items = ((gp.n + 255) / 256) * max_tiles, slices = (gp.K + 63) / 64, step = WideShapeT<FMT>::kChunkSlices;
+            const int most = std::min(plan->sm_count, kSplitCtas) / items;
+            double least = slices;
+            for (int want = 2; want <= most; want++) {
+                const int per = ((slices + want - 1) / want + step - 1) / step * step, n = (slices + per - 1) / per;
+                const double cost = per + 4.0 + (double)n * gp.dense_rows * gp.n * 8.0 / 4e6;
+                if (n > 1 && cost < least) { least = cost; gp.splits = n; gp.split_slices = per; }
+            }
+            if (gp.splits > 1) {
+                uint16_t* out = gp.out;
+                gp.partial = plan->ws.split_partial;
+                ALLOW_SMEM_ONCE((grouped_gemm_wide_kernel<FMT, kEpiPartialF32>));
+                CK(launch_dependent(grouped_gemm_wide_kernel<FMT, kEpiPartialF32>, dim3(items * gp.splits), dim3(WideShapeT<FMT>::kThreads),
+                                    WideShapeT<FMT>::kSmemBytes, st, gp, maps[0], maps[1], maps[2], maps[3]));
+                const size_t total = (size_t)gp.dense_rows * gp.n;
+                CK(launch_dependent(split_sum_kernel, dim3((unsigned)((total / 4 + 255) / 256)), dim3(256), 0, st, gp.partial, gp.splits, total, out));
+                plan->launches += 2;
+                CK(cudaGetLastError());
+                return OCO_OK;
+            }
+        }
     }
     ALLOW_SMEM_ONCE((grouped_gemm_wide_kernel<FMT, EPI>));
     // persistent: one CTA per SM walks the (route tile, feature tile) items; never more CTAs than items can exist

@@ -31,7 +31,8 @@ enum GemmEpilogue : int {
     kEpiSiluF16 = 1,    // gated, SiLU gate over bf16-rounded projections -> half rows
     kEpiRelu2F16 = 2,   // bf16-rounded projection, relu^2 in f32 -> half rows
     kEpiDownBf16 = 3,   // (+ bias) -> bf16, scattered to each route's row
-    kEpiRelu2Bf16F16 = 4  // dense shared expert: relu^2 stored as bf16, then to half
+    kEpiRelu2Bf16F16 = 4, // dense shared expert: relu^2 stored as bf16, then to half
+    kEpiPartialF32 = 5    // dense, a part of the contraction: f32 sums for split_sum_kernel (wide kernel only)
 };
 __host__ __device__ constexpr bool epi_gated(int epi) { return epi == kEpiSwigluF16 || epi == kEpiSiluF16; }
 
@@ -62,6 +63,8 @@ struct GemmParams {
     int sfa_tiles;             //   feature tiles per expert
     uint32_t* sched;           // wide kernel: two zeroed words (items handed out, CTAs finished) for handing out work
                                //   items as CTAs become free; null = item c, c + grid, ... for CTA c
+    int splits, split_slices;  // kEpiPartialF32: parts of the contraction, and 64-wide K slices in each
+    float* partial;            //   [splits][dense_rows][n]
 };
 
 // ---- operand order ---------------------------------------------------------------------------------

@@ -93,10 +93,16 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
     // ---- the work list ---------------------------------------------------------------------------
     const int nfeat = (p.n + kFeatPerItem - 1) / kFeatPerItem;
     const int ntiles = p.tiles ? (int)*p.tile_count : (p.dense_rows + NT - 1) / NT;
-    const int total = nfeat * ntiles;
-    struct Item { uint32_t expert, row0, nv; int f0; };
+    constexpr bool SPLIT = EPI == kEpiPartialF32;                      // the list runs once per part of the contraction
+    const int nkb = (p.K + 63) / 64;
+    const int total = nfeat * ntiles * (SPLIT ? p.splits : 1);
+    struct Item { uint32_t expert, row0, nv; int f0, kb0, kb1, split; };
     auto load_item = [&](int item) {
         Item r;
+        r.split = SPLIT ? item / (nfeat * ntiles) : 0;
+        r.kb0 = SPLIT ? r.split * p.split_slices : 0;
+        r.kb1 = SPLIT ? min(nkb, r.kb0 + p.split_slices) : nkb;
+        if (SPLIT) item -= r.split * nfeat * ntiles;
         const int tile = item / nfeat;
         r.f0 = (item - tile * nfeat) * kFeatPerItem;
         uint32_t begin, count;
@@ -111,7 +117,6 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         r.nv = min((uint32_t)NT, count - begin);
         return r;
     };
-    const int nkb = (p.K + 63) / 64;
     const int nblk = p.K >> 5;
 
     // ---- shared memory carve-up ----------------------------------------------------------------
@@ -168,7 +173,8 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         constexpr int NC = S::kCopies;
         constexpr uint32_t kBufBytes = 16 * S::kPitch;
         const uint32_t ring = ring_base + (uint32_t)warp * S::kRingWarp;
-        const int nchunks = (nkb + S::kChunkSlices - 1) / S::kChunkSlices;
+        int chunk0 = 0, nchunks = (nkb + S::kChunkSlices - 1) / S::kChunkSlices;   // ring chunks [chunk0, nchunks) of an item
+        int g_run = 0;                                                         // slices of earlier items
         // packed bytes of tile row trow0 + r of an item
         auto row_ptr = [&](const Item& it, int r) -> const uint8_t* {
             const int feat0 = GATED ? it.f0 : it.f0 + 128 * tile;
@@ -220,20 +226,28 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         if (fetcher) { item_slot[0] = blockIdx.x; mbar_arrive(item_full(0)); }
         // the chunk during which the fetcher asks for the CTA's next item: late, so that a CTA holds no item it
         // will not start soon, yet a few slices before the end, so that the answer is there when the item ends
-        const int fetch_chunk = max(0, nchunks - 4);
+        const int fetch_chunk = SPLIT ? -1 : max(0, nchunks - 4);
         uint32_t fetched = 0;
         int next = 0;
         for (int item = blockIdx.x; item < total; item = next, seq++) {
             if (!started) {
                 cur = load_item(item);
+                if (SPLIT) { chunk0 = cur.kb0 / S::kChunkSlices; nchunks = (cur.kb1 + S::kChunkSlices - 1) / S::kChunkSlices; }
 #pragma unroll
                 for (int i = 0; i < NC; i++) csrc[i] = row_ptr(cur, crow[i]);
-                issue(csrc, 0);
+                issue(csrc, chunk0);
             }
             const uint32_t a_lo = (uint32_t)(uintptr_t)row_ptr(cur, r) & 15u;   // alignment of the row start
-            const int g0 = seq * nkb;                                           // slices of earlier items
-            for (int chunk = 0; chunk < nchunks; chunk++) {
+            const int g0 = SPLIT ? g_run - cur.kb0 : seq * nkb;                  // slices of earlier items (less the first of this)
+            if (SPLIT) {
+                g_run += cur.kb1 - cur.kb0;
                 if (fetcher) {
+                    item_slot[(seq + 1) & 1] = min((uint32_t)item + gridDim.x, (uint32_t)total);
+                    mbar_arrive(item_full((seq + 1) & 1));
+                }
+            }
+            for (int chunk = chunk0; chunk < nchunks; chunk++) {
+                if (!SPLIT && fetcher) {
                     if (chunk == fetch_chunk) fetched = dyn ? gridDim.x + atomicAdd(p.sched, 1u) : (uint32_t)item + gridDim.x;
                     if (chunk == min(fetch_chunk + 2, nchunks - 1)) {
                         item_slot[(seq + 1) & 1] = min(fetched, (uint32_t)total);
@@ -258,7 +272,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
 #pragma unroll
                 for (int kk = 0; kk < S::kChunkSlices; kk++) {
                     const int kb = chunk * S::kChunkSlices + kk;
-                    if (kb < nkb) {
+                    if (kb < (SPLIT ? cur.kb1 : nkb)) {
                         uint32_t v[16];
                         if (SUPER) {
                             // code bytes 16 h .. 16 h + 15 of the slice's sub-block pair
@@ -306,9 +320,10 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
             started = next < total;
             if (started) {
                 cur = load_item(next);
+                if (SPLIT) { chunk0 = cur.kb0 / S::kChunkSlices; nchunks = (cur.kb1 + S::kChunkSlices - 1) / S::kChunkSlices; }
 #pragma unroll
                 for (int i = 0; i < NC; i++) csrc[i] = row_ptr(cur, crow[i]);
-                issue(csrc, 0);
+                issue(csrc, chunk0);
             }
             // ===== epilogue of `done` ================================================================
             asm volatile("bar.sync 1, %0;" ::"n"(S::kProducerWarps * 32) : "memory");                    // nobody still reads the row map of the item before
@@ -342,10 +357,13 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     if (c + j < done.nv) {
-                        const size_t orow = (size_t)out_rows[c + j] * p.n;
+                        const size_t orow = ((SPLIT ? (size_t)done.split * p.dense_rows : 0) + out_rows[c + j]) * p.n;
                         const float a = __fadd_rn(__uint_as_float(ra[j]), bias_a);
                         const float b = __fadd_rn(__uint_as_float(rb[j]), bias_b);
-                        if (GATED) {
+                        if (SPLIT) {
+                            if (fa < p.n) p.partial[orow + fa] = a;
+                            if (fb < p.n) p.partial[orow + fb] = b;
+                        } else if (GATED) {
                             if (fa < p.n) p.out[orow + col_a] = epilogue_value<EPI>(a, b);
                         } else {
                             if (fa < p.n) p.out[orow + col_a] = epilogue_value<EPI>(a, 0.f);
@@ -363,7 +381,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
     } else if (warp == S::kMmaWarp) {
         if (lane == 0) {
             // ===== MMA issue ======================================================================
-            int seq = 0;
+            int seq = 0, g_run = 0;
             for (int item = item_of(0); item < total; item = item_of(++seq)) {
                 const Item it = load_item(item);
                 const uint32_t n_mma = max(16u, (it.nv + 15u) & ~15u);
@@ -372,8 +390,9 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                     mbar_wait(tmem_free, (uint32_t)(seq - 1) & 1u, abort_flag, p.status);
                     tc_fence_after();
                 }
-                const int g0 = seq * nkb;
-                for (int kb = 0; kb < nkb; kb++) {
+                const int g0 = SPLIT ? g_run - it.kb0 : seq * nkb;
+                if (SPLIT) g_run += it.kb1 - it.kb0;
+                for (int kb = it.kb0; kb < it.kb1; kb++) {
                     const int g = g0 + kb, sa = g % S::kAStages, sb = g % S::kBStages;
                     mbar_wait(full_a(sa), (uint32_t)(g / S::kAStages) & 1u, abort_flag, p.status);
                     mbar_wait(full_b(sb), (uint32_t)(g / S::kBStages) & 1u, abort_flag, p.status);
@@ -383,7 +402,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                     const uint64_t b = umma_desc(b_base + (uint32_t)sb * S::kBStage);
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
-                        const uint32_t acc = (kb | kk) != 0 ? 1u : 0u;
+                        const uint32_t acc = ((kb - it.kb0) | kk) != 0 ? 1u : 0u;
                         umma_f16(tmem_base, a0 + 2u * kk, b + 2u * kk, idesc, acc);
                         umma_f16(tmem_base + NT, a1 + 2u * kk, b + 2u * kk, idesc, acc);
                     }
@@ -397,14 +416,15 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         }
     } else if (lane == 0) {
         // ===== B tiles by TMA =========================================================================
-        int seq = 0;
+        int seq = 0, g_run = 0;
         for (int item = item_of(0); item < total; item = item_of(++seq)) {
             const Item it = load_item(item);
-            const int g0 = seq * nkb;
+            const int g0 = SPLIT ? g_run - it.kb0 : seq * nkb;
+            if (SPLIT) g_run += it.kb1 - it.kb0;
             // the smallest box (32, 64, 128 or 256 rows of 64 halves) that holds the tile's live rows
             const CUtensorMap* box = it.nv <= 32 ? &tmap_b32 : it.nv <= 64 ? &tmap_b64 : it.nv <= 128 ? &tmap_b128 : &tmap_b;
             const uint32_t box_bytes = (it.nv <= 32 ? 32u : it.nv <= 64 ? 64u : it.nv <= 128 ? 128u : 256u) * 128u;
-            for (int kb = 0; kb < nkb; kb++) {
+            for (int kb = it.kb0; kb < it.kb1; kb++) {
                 const int g = g0 + kb, sb = g % S::kBStages;
                 mbar_wait(empty_b(sb), ((uint32_t)(g / S::kBStages) & 1u) ^ 1u, abort_flag, p.status);
                 mbar_arrive_expect_tx(full_b(sb), box_bytes);
@@ -422,6 +442,29 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         tmem_dealloc(tmem_base, S::kTmemCols);
     }
     leave();
+}
+
+// Adds the parts of a split dense product in order and stores bf16. total = rows * n, a multiple of four; a thread
+// takes four outputs of neighbouring features. Bound by reading the partial sums (from L2, where they were just
+// written).
+__global__ void __launch_bounds__(256) split_sum_kernel(const float* __restrict__ partial, int splits, size_t total, uint16_t* __restrict__ out) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
+    if (i >= total) return;
+    float4 v = *reinterpret_cast<const float4*>(partial + i);
+#pragma unroll 4
+    for (int s = 1; s < splits; s++) {
+        const float4 u = *reinterpret_cast<const float4*>(partial + (size_t)s * total + i);
+        v.x = __fadd_rn(v.x, u.x); v.y = __fadd_rn(v.y, u.y); v.z = __fadd_rn(v.z, u.z); v.w = __fadd_rn(v.w, u.w);
+    }
+    const uint16_t h[4] = {epilogue_value<kEpiDownBf16>(v.x, 0.f), epilogue_value<kEpiDownBf16>(v.y, 0.f), epilogue_value<kEpiDownBf16>(v.z, 0.f),
+                           epilogue_value<kEpiDownBf16>(v.w, 0.f)};
+    if (((uintptr_t)out & 7u) == 0) {
+        *reinterpret_cast<uint2*>(out + i) = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
+    } else {
+        for (int q = 0; q < 4; q++) out[i + q] = h[q];
+    }
 }
 
 }  // namespace oco

@@ -91,6 +91,34 @@ def test_mxfp4_projection_at_the_gpt_oss_width(dense, oracle):
         check(dense, oracle, dense.PROJECTION, synth.FMT_MXFP4, 2880, 2880, rows, 21)
 
 
+@pytest.mark.parametrize("fmt,H,F,rows", [(synth.FMT_Q4_0, 2080, 320, 33), (synth.FMT_MXFP4, 2912, 288, 300), (synth.FMT_Q4_K, 2304, 544, 257),
+                                          (synth.FMT_Q4_K, 7936, 32, 700), (synth.FMT_Q4_0, 8224, 64, 16)])
+def test_projection_over_a_split_contraction(dense, oracle, fmt, H, F, rows):
+    """Few items and a long contraction: parts of unequal length, a last K slice that is half full, partial tiles of
+    features and rows. (Too short a contraction, or enough items, stays whole: the shapes above.)"""
+    check(dense, oracle, dense.PROJECTION, fmt, H, F, rows, 60 + rows, x_scale=0.25)
+
+
+def test_split_contraction_stores_to_any_output_address(dense, oracle):
+    import torch
+    H, F, rows = 2080, 320, 40
+    rng = np.random.default_rng(5)
+    up_w = synth.random_q4_0(rng, F, H)
+    x_bits, _ = synth.make_tokens(H, rows, 6, "zero")
+    plan = dense.DensePlan(dense.PROJECTION, synth.FMT_Q4_0, H, F)
+    plan.reserve(rows)
+    plan.bind(up_w, None, None)
+    x = torch.from_numpy(x_bits.view(np.int16)).cuda()
+    outs = []
+    for skip in (0, 1):
+        y = torch.full((rows * F + 2,), 77, dtype=torch.int16, device="cuda")
+        plan.forward(x, y[skip:skip + rows * F], rows)
+        torch.cuda.synchronize()
+        assert bool((y[:skip] == 77).all()) and bool((y[skip + rows * F:] == 77).all())
+        outs.append(y[skip:skip + rows * F].cpu().numpy())
+    assert np.array_equal(outs[0], outs[1])
+
+
 def test_unsupported_pairs_and_bad_calls_are_refused(dense):
     from oco_b200 import _lib
     from oco_b200.moe import OcoError
