@@ -8,8 +8,8 @@
 //
 //   route_plan_kernel (tile_rows = 8)  ->  groups of up to 8 routes of one expert
 //   batch_fragments_kernel             ->  each group's token rows as B fragments
-//   batch_expand_kernel                ->  activations (half, expert-sorted) + the down stage's fragments
-//   batch_down_kernel                  ->  bf16 expert outputs in route order
+//   batch_rows_kernel, up epilogue     ->  activations (half, expert-sorted) + the down stage's fragments
+//   batch_rows_kernel, down epilogue   ->  bf16 expert outputs in route order
 #pragma once
 #include "decode.cuh"
 #include "gemm.cuh"
