@@ -111,7 +111,7 @@ struct BatchParams {
 // (or fewer) the last wave decided: 19 groups made 152 CTAs of three rounds on 148 SMs, six rounds where three
 // suffice. Within its run a warp starts the next unit's first stage under the last stage of the one before, across
 // groups too, so that its rows never stop; only the group's fragments are waited for when the group changes.
-// gpt-oss-20b-shaped step of 7 tokens 177 -> 137 us, 120b-shaped one of 64 tokens 517 -> 494 us. Qwen3 (Q4_K), which
+// gpt-oss-20b-shaped step of 7 tokens 156 -> 139 us (179 -> 139 with other routes), 120b-shaped one of 64 tokens 561 -> 492 us. Qwen3 (Q4_K), which
 // took 256-route tiles for any batch: 2 rows 136 -> 66 us, 8 rows 352 -> 130, 32 rows 254 -> 200, 96 rows 306 -> 250.
 template <int FMT, int EPI>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_rows_kernel(const BatchParams p) {
