@@ -432,7 +432,8 @@ int launch_gemm_wide(oco_moe_plan* plan, GemmParams gp, const CUtensorMap* maps,
                 CK(launch_dependent(grouped_gemm_wide_kernel<FMT, kEpiPartialF32>, dim3(items * gp.splits), dim3(WideShapeT<FMT>::kThreads),
                                     WideShapeT<FMT>::kSmemBytes, st, gp, maps[0], maps[1], maps[2], maps[3]));
                 const size_t total = (size_t)gp.dense_rows * gp.n;
-                CK(launch_dependent(split_sum_kernel, dim3((unsigned)((total / 4 + 255) / 256)), dim3(256), 0, st, gp.partial, gp.splits, total, out));
+                CK(launch_dependent(split_sum_kernel, dim3((unsigned)((total / 4 + 255) / 256)), dim3(256), 0, st, gp.partial, gp.splits, total, out,
+                                    gp.status));
                 plan->launches += 2;
                 CK(cudaGetLastError());
                 return OCO_OK;

@@ -446,10 +446,13 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
 
 // Adds the parts of a split dense product in order and stores bf16. total = rows * n, a multiple of four; a thread
 // takes four outputs of neighbouring features. Bound by reading the partial sums (from L2, where they were just
-// written).
-__global__ void __launch_bounds__(256) split_sum_kernel(const float* __restrict__ partial, int splits, size_t total, uint16_t* __restrict__ out) {
+// written). Once a wait has given up, the parts are not those of this call (the tile kernel leaves at its start): the
+// output then stays as it was.
+__global__ void __launch_bounds__(256) split_sum_kernel(const float* __restrict__ partial, int splits, size_t total, uint16_t* __restrict__ out,
+                                                        const uint32_t* status) {
     pdl_launch_dependents();
     pdl_wait();
+    if (*reinterpret_cast<const volatile uint32_t*>(status) != 0u) return;
     const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
     if (i >= total) return;
     float4 v = *reinterpret_cast<const float4*>(partial + i);

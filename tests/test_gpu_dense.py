@@ -119,6 +119,34 @@ def test_split_contraction_stores_to_any_output_address(dense, oracle):
     assert np.array_equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("H,F,rows", [(2080, 320, 40), (320, 4096, 300)], ids=["split", "whole"])
+def test_a_step_after_a_wait_that_gave_up_leaves_the_output(dense, oracle, H, F, rows):
+    """While the status word (the workspace's first) is set, a product writes nothing of its own or of an earlier call
+    to the output; poll reports it once, and the next call is right again."""
+    import torch
+    from oco_b200 import _lib
+    from oco_b200.moe import OcoError
+    up_w = synth.random_q4_0(np.random.default_rng(8), F, H)
+    plan = dense.DensePlan(dense.PROJECTION, synth.FMT_Q4_0, H, F)
+    plan.reserve(rows)
+    plan.bind(up_w, None, None)
+    x_bits, _ = synth.make_tokens(H, rows, 6, "zero")
+    x = torch.from_numpy(x_bits.view(np.int16)).cuda()
+    y, again = (torch.full((rows, F), 77, dtype=torch.int16, device="cuda") for _ in range(2))
+    plan.forward(x, y, rows)                       # leaves its parts in the workspace
+    plan.poll()
+    want = y.clone()
+    plan.workspace[:4].view(torch.int32).fill_(1)  # what a wait that gives up leaves there
+    plan.forward(x, again, rows)
+    with pytest.raises(OcoError) as e:
+        plan.poll()
+    assert e.value.code == _lib.DEVICE_TIMEOUT
+    assert bool((again == 77).all()), "a step after a wait that gave up wrote its output"
+    plan.forward(x, again, rows)
+    plan.poll()
+    assert torch.equal(again, want)
+
+
 def test_unsupported_pairs_and_bad_calls_are_refused(dense):
     from oco_b200 import _lib
     from oco_b200.moe import OcoError
