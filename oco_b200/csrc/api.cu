@@ -834,9 +834,10 @@ int stage_experts(oco_moe_plan* plan, const uint16_t* x, const uint32_t* ids, in
     const int H = d.hidden, F = d.ffn, E = d.experts;
     const int live = rs.expected > 0 && rs.expected < R ? rs.expected : R;   // routes expected to carry this plan's experts
     if (d.numerics == 0 && live <= plan->batch_max_avg * E && (rs.expected == 0 || R <= 64 * E) && !plan->no_batch_path &&
-        batch_smem_bytes(FMT, H / 32) <= kMaxDynamicSmem && batch_smem_bytes(FMT, F / 32) <= kMaxDynamicSmem) {
+        batch_smem_bytes(FMT, H / 32) <= kMaxDynamicSmem && batch_smem_bytes(FMT, F / 32) <= kMaxDynamicSmem && ((uintptr_t)x & 7u) == 0) {
         // A few routes per expert: memory-bound, streamed with up to eight routes per MMA (batch.cuh).
-        // (Layers too wide for the fragments to sit in shared memory take the tiles.)
+        // (Layers too wide for the fragments to sit in shared memory take the tiles, and so do rows that do not start on
+        // eight bytes, which oco_moe_experts may be given: batch_fragments_kernel reads four values at once.)
         {
             plan->last_tile_rows = kBatchCols;
             launch_route_plan(plan, ids, R, E, kBatchCols, rs, st);

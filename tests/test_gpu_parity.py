@@ -778,6 +778,46 @@ def test_expert_shard_with_fewer_experts_than_routes_per_token(moe, oracle):
 
 
 
+@pytest.mark.parametrize("arch,fmt", [(synth.ARCH_GPT_OSS, synth.FMT_MXFP4), (synth.ARCH_NEMOTRON, synth.FMT_Q4_0), (synth.ARCH_QWEN, synth.FMT_Q4_K)],
+                         ids=["gpt-oss", "nemotron", "qwen"])
+def test_expert_rows_at_any_address_take_a_kernel_that_reads_them(moe, arch, fmt, monkeypatch):
+    """oco_moe_experts with a few routes per expert and rows that start on two or four bytes: they go through the tile
+    kernels, whose gather reads element by element where it has to, and give the bits that aligned rows give there."""
+    import ctypes as C
+    import torch
+    from oco_b200 import _lib
+    E, H, F, R = 8, 256, 256, 20
+    layer = synth.make_layer(arch, H, F, E, 2, fmt, seed=29)
+    x, _ = synth.make_tokens(H, R, 3)
+    x = torch.from_numpy(synth.f32_to_bf16_bits(synth.bf16_bits_to_f32(x) * np.float32(0.25)).view(np.int16)).cuda()
+    ids = torch.from_numpy(np.random.default_rng(1).integers(0, E, size=R).astype(np.int32)).cuda()
+
+    def experts(plan, skip):
+        room = torch.zeros(R * H + 8, dtype=torch.int16, device="cuda")
+        rows, y = room[skip:skip + R * H], torch.zeros((R, H), dtype=torch.int16, device="cuda")
+        rows.copy_(x.reshape(-1))
+        rc = _lib.lib().oco_moe_experts(plan.handle, C.c_void_p(rows.data_ptr()), C.c_void_p(ids.data_ptr()), R, C.c_void_p(y.data_ptr()),
+                                        C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == _lib.OK, _lib.lib().oco_moe_last_error(plan.handle)
+        plan.poll()
+        return y
+
+    def planned():
+        plan = moe.plan_for(layer)
+        plan.reserve(R)
+        plan.bind(moe._Weights.from_layer(layer))
+        return plan
+
+    streamed = planned()
+    monkeypatch.setenv("OCO_MOE_NO_BATCH", "1")
+    want = experts(planned(), 0)
+    for skip in (1, 2):
+        assert torch.equal(experts(streamed, skip), want)
+    close = experts(streamed, 4)                # eight bytes are enough for the streamed kernels
+    err = rel_l2(close.cpu().numpy().view(np.uint16), want.cpu().numpy().view(np.uint16))
+    assert err <= REL_L2
+
+
 # ---- opt-in block-scaled numerics (numerics = 2): MXFP4 activations on tcgen05 kind::mxf4 ---------------
 def _swiglu(gate, up):
     g = np.minimum(gate, 7.0)
