@@ -18,10 +18,10 @@
 #include "gemm_pair.cuh"
 #include "mx.cuh"
 #include "gemm_mx.cuh"
-#include <climits>
 #include <cmath>
 #include "plan.cuh"
 #include "router.cuh"
+#include "token_deal.h"
 
 using namespace oco;
 
@@ -467,27 +467,6 @@ int launch_gemm_nt(oco_moe_plan* plan, const GemmParams& gp, const CUtensorMap* 
     }
 }
 
-// Warps per unit of the single-token kernels: as many as keep every warp of the grid busy.
-int pick_ksplit(int units, int ctas, int warps_per_cta) {
-    for (int k : {10, 8, 5, 4, 2})
-        if (warps_per_cta % k == 0 && units * k <= ctas * warps_per_cta) return k;
-    return 1;
-}
-
-// The same where the units are more than half the warps (routed and always-on expert in one launch): the split with
-// the fewest blocks in a row for the busiest warp, several rounds of units allowed. At 928 units of 84 blocks on 148
-// x 20 warps two warps per unit leave a third of the warps without one (42 blocks in a row), five take 34.
-int pick_ksplit_rounds(int units, int nkb, int ctas, int warps_per_cta) {
-    int best = 1, least = INT_MAX;
-    for (int k : {1, 2, 4, 5, 8, 10}) {
-        if (warps_per_cta % k) continue;
-        const int slots = ctas * (warps_per_cta / k), rounds = (units + slots - 1) / slots, run = rounds * ((nkb + k - 1) / k);
-        if (run < least) { least = run; best = k; }
-    }
-    return best;
-}
-
-
 template <int ARCH, int FMT>
 int launch_expand(oco_moe_plan* plan, DecodeExpandParams ep, cudaStream_t st) {
     const int grid = plan->sm_count;
@@ -506,13 +485,9 @@ int launch_down(oco_moe_plan* plan, DecodeDownParams dp, cudaStream_t st) {
     const int grid = plan->sm_count;
     const int widest = std::max(dp.F, dp.sh_F);
     if (token_smem_bytes(FMT, widest / 32, 2) > kMaxDynamicSmem) return fail(plan, OCO_UNSUPPORTED_SHAPE, "expert width %d too large for the single-token kernels", widest);
-    // the always-on expert gets CTAs in proportion to its width
-    dp.sh_shares = dp.sh_F ? std::max(1, (dp.sh_F + dp.F / 2) / dp.F) : 0;
-    if (dp.K + dp.sh_shares > grid) dp.sh_shares = dp.sh_F ? 1 : 0;
-    const int places = dp.K + dp.sh_shares;
-    if (places > grid) return fail(plan, OCO_UNSUPPORTED_SHAPE, "more routes than multiprocessors");
-    dp.ksplit = pick_ksplit(dp.H / 16, grid / places, tok_warps(FMT));
-    dp.sh_ksplit = dp.sh_F ? pick_ksplit(dp.H / 16, grid / places * dp.sh_shares, tok_warps(FMT)) : 1;
+    const DownDeal deal = deal_down(dp.K, dp.H / 16, dp.F / 32, dp.sh_F / 32, grid, tok_warps(FMT));
+    if (!deal.turns) return fail(plan, OCO_UNSUPPORTED_SHAPE, "more routes than multiprocessors");
+    dp.sh_shares = deal.shares; dp.ksplit = deal.ksplit; dp.sh_ksplit = deal.sh_ksplit;
     ALLOW_SMEM_ONCE((decode_down_kernel<FMT, 2>));
     CK(launch_dependent(decode_down_kernel<FMT, 2>, dim3(grid), dim3(tok_warps(FMT) * 32), token_smem_bytes(FMT, widest / 32, 2), st, dp));
     plan->launches++;

@@ -504,9 +504,10 @@ def test_few_tokens_equal_shares(moe, oracle, arch, hidden, ffn, experts, top_k,
     check_layer(moe, oracle, layer, tokens, seed=tokens + 1, misalign=5)
 
 
-@pytest.mark.parametrize("ffn,shared_ffn,top_k", [(192, 64, 6), (160, 1920, 2), (96, 96, 6), (64, 4096, 1)])
+@pytest.mark.parametrize("ffn,shared_ffn,top_k", [(192, 64, 6), (160, 1920, 2), (96, 96, 6), (64, 4096, 1), (32, 4800, 6), (64, 4416, 6)])
 def test_nemotron_single_token_always_on_expert(moe, oracle, ffn, shared_ffn, top_k):
-    """The always-on expert in the routed launches: narrower than, as wide as and much wider than a routed one."""
+    """The always-on expert in the routed launches: narrower than, as wide as and much wider than a routed one, up to
+    where its part of the CTAs is no longer in proportion to its width."""
     layer = synth.make_layer(synth.ARCH_NEMOTRON, 352, ffn, 16, top_k, synth.FMT_Q4_0, seed=ffn, shared_ffn=shared_ffn, normalize=True, scale=2.5)
     check_layer(moe, oracle, layer, 1, seed=ffn, residual="normal")
     check_layer(moe, oracle, layer, 1, seed=ffn + 1, misalign=7)

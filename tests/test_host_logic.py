@@ -138,3 +138,54 @@ def test_window_geometry_and_labels():
         assert np.array_equal(lab, src * sr + r)
         assert np.array_equal(lab // top_k, src * st + r // top_k)      # the token's row in the token window
         assert len(np.unique(lab)) == len(lab)
+
+
+@pytest.fixture(scope="module")
+def token_deal(tmp_path_factory):
+    """The host rules that deal out the single-token kernels' units, compiled by themselves."""
+    import ctypes as C
+    import os
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "oco_b200", "csrc")
+    work = tmp_path_factory.mktemp("deal")
+    (work / "deal.cpp").write_text('#include "token_deal.h"\n'
+                                   'extern "C" void deal_down(int k, int rows, int nkb, int sh, int ctas, int warps, int* out) {\n'
+                                   '    const oco::DownDeal d = oco::deal_down(k, rows, nkb, sh, ctas, warps);\n'
+                                   '    out[0] = d.shares; out[1] = d.turns; out[2] = d.ksplit; out[3] = d.sh_ksplit;\n}\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", csrc, "-o", str(work / "deal.so"), str(work / "deal.cpp")], check=True)
+    fn = C.CDLL(str(work / "deal.so")).deal_down
+
+    def deal(k, hidden, ffn, shared, ctas=148, warps=20):
+        out = (C.c_int * 4)()
+        fn(k, hidden // 16, ffn // 32, shared // 32, ctas, warps, out)
+        return tuple(out)
+    return deal
+
+
+def _blocks_in_a_row(rows, nkb, ctas, warps, ksplit):
+    return -(-rows // (ctas * (warps // ksplit))) * (-(-nkb // ksplit) + 16)
+
+
+@pytest.mark.parametrize("k,hidden,ffn,shared", [(6, 2688, 1856, 3712), (6, 2688, 32, 4800), (6, 4096, 64, 4416), (1, 352, 64, 4096), (8, 2688, 1856, 7424),
+                                                 (6, 2688, 1856, 32), (8, 256, 32, 64)])
+def test_always_on_expert_gets_its_part_of_the_ctas(token_deal, k, hidden, ffn, shared):
+    """Down launch of a single token: every place has a CTA, and no number of shares would leave the busiest warp less to do (blocks
+    in a row, and sixteen for the start of each unit): an always-on expert 150 times as wide as a routed one had a seventh
+    of the CTAs, and one 69 times as wide left each route a single CTA."""
+    def run(shares, turns, ksplit, sh_ksplit):
+        return max(_blocks_in_a_row(hidden // 16, ffn // 32, turns, 20, ksplit),
+                   _blocks_in_a_row(hidden // 16, shared // 32, turns * shares, 20, sh_ksplit))
+
+    shares, turns, ksplit, sh_ksplit = token_deal(k, hidden, ffn, shared)
+    assert shares >= 1 and turns >= 1 and (k + shares) * turns <= 148
+    pick = lambda units, ctas: next((q for q in (10, 5, 4, 2) if units * q <= ctas * 20), 1)
+    every = [run(s, 148 // (k + s), pick(hidden // 16, 148 // (k + s)), pick(hidden // 16, 148 // (k + s) * s)) for s in range(1, 149 - k)]
+    assert run(shares, turns, ksplit, sh_ksplit) == min(every)
+
+
+def test_down_deal_at_its_limits(token_deal):
+    assert token_deal(4, 2880, 2880, 0) == (0, 37, 4, 1)             # no always-on expert: a place for each route
+    assert token_deal(6, 2688, 1856, 3712)[:2] == (2, 18)            # a Nemotron-H layer: twice the width, twice the CTAs
+    assert token_deal(8, 256, 256, 0, ctas=7)[1] == 0                # more routes than CTAs: refused by the launch
+    assert token_deal(8, 256, 256, 256, ctas=8)[1] == 0
+    assert token_deal(8, 256, 256, 256, ctas=9)[:2] == (1, 1)
