@@ -58,7 +58,6 @@ struct Workspace {
     uint16_t* shared_out = nullptr;  // bf16 [T, H]
     float* sh_act1 = nullptr;
     __half* sh_actfrag = nullptr;
-    uint32_t* sh_ids = nullptr;
     uint16_t* norm = nullptr;     // bf16 [T, H] normalised rows of oco_moe_add_norm_forward
     unsigned char* mx_xb = nullptr;   // block-scaled single-token path: the token as e2m1 pieces
     unsigned char* mx_xsfb = nullptr; //   and their scales
@@ -88,6 +87,7 @@ struct oco_moe_plan {
     int sm_count = 148;
     int launches = 0;
     int last_tile_rows = 0;
+    int split_width = 0;         // output features of the dense product whose contraction may be split (0: the plan has none)
     uint32_t up_row_bytes = 0, down_row_bytes = 0, shared_up_row_bytes = 0, shared_down_row_bytes = 0;
     // Resolved gate / up operands: two tensors, or the rows of one interleaved tensor (row 2c = gate c,
     // row 2c + 1 = up c), in which case consecutive rows of either matrix lie two packed rows apart.
@@ -193,14 +193,15 @@ int block_elems(int fmt) { return fmt == OCO_FMT_Q4_K ? 256 : 32; }
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Lays the workspace out; with base == nullptr only the total is meaningful.
-// Route groups (up to eight routes of one expert) that R routes over E experts can form.
 // CTAs that a split dense product may use, whatever the GPU has: bounds its partial sums in the workspace.
 constexpr int kSplitCtas = 148;
 
+// Route groups (up to eight routes of one expert) that R routes over E experts can form.
 size_t batch_max_groups(size_t R, size_t E) { return R / 8 + (E < R ? E : R); }
 
-Workspace carve(const oco_moe_desc& d, int max_rows, unsigned char* base) {
+// Lays the workspace out; with base == nullptr only the total is meaningful. split_width: output features of the
+// product that may be split over its contraction (0: none).
+Workspace carve(const oco_moe_desc& d, int split_width, int max_rows, unsigned char* base) {
     Workspace w;
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -240,16 +241,11 @@ Workspace carve(const oco_moe_desc& d, int max_rows, unsigned char* base) {
         w.shared_out = (uint16_t*)take(T * H * 2);
         w.sh_act1 = (float*)take(S * 4);
         w.sh_actfrag = (__half*)take((S / 32) * 128 * 2);
-        w.sh_ids = (uint32_t*)take(256);
     }
-    if (S || (E == 1 && d.numerics == 0)) {
-        // partial sums of a split dense product: at most kSplitCtas items of 256 x 256 outputs
-        auto parts = [&](size_t n) {
-            const size_t most = (size_t)kSplitCtas / ((n + 255) / 256);
-            return most < 2 ? (size_t)0 : std::min((size_t)kSplitCtas * 256 * 256, most * T * n);
-        };
-        const size_t floats = std::max(parts(H), parts(F));
-        if (floats) w.split_partial = (float*)take(floats * 4);
+    if (split_width) {
+        // partial sums of the split product: at most kSplitCtas items of 256 x 256 outputs, parts of T rows each
+        const size_t n = (size_t)split_width, most = (size_t)kSplitCtas / ((n + 255) / 256);
+        if (most >= 2) w.split_partial = (float*)take(std::min((size_t)kSplitCtas * 256 * 256, most * T * n) * 4);
     }
     w.norm = (uint16_t*)take(T * H * 2);
     if (d.weight_format == OCO_FMT_MXFP4) {
@@ -320,6 +316,9 @@ int make_byte_map(oco_moe_plan* plan, CUtensorMap* map, void* base, uint64_t row
     if (r != CUDA_SUCCESS) return fail(plan, OCO_CUDA_ERROR, "cuTensorMapEncodeTiled (byte rows) failed (%d)", (int)r);
     return OCO_OK;
 }
+
+// Only the wide tile kernel splits a contraction; a plan that was asked for the generic kernels never reaches it.
+bool split_tiles(const oco_moe_plan* plan) { return plan->d.gemm_impl == 0 && !plan->narrow_tiles; }
 
 // Route-tile height by the average number of routes per expert. Layers take the 256-route tiles of
 // the wide kernel from `wide_min_avg` routes per expert on (its cost per tile hardly depends on the
@@ -1062,6 +1061,7 @@ int oco_moe_plan_create(const oco_moe_desc* desc, oco_moe_plan** out) {
     // 305 us, 128 rows (8) 312 | 307.
     if (d.weight_format == OCO_FMT_Q4_K) plan->batch_max_avg = 6;
     { const char* e = getenv("OCO_MOE_BATCH_MAX_AVG"); if (e && atoi(e) > 0) plan->batch_max_avg = atoi(e) < 64 ? atoi(e) : 64; }
+    plan->split_width = split_tiles(plan) && d.shared_ffn ? d.hidden : 0;      // the always-on expert's down product
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
@@ -1108,13 +1108,13 @@ int oco_moe_phase_times(oco_moe_plan* plan, int capacity, float* ms, const char*
 
 size_t oco_moe_workspace_bytes(const oco_moe_plan* plan, int max_rows) {
     if (!plan || max_rows < 1) return 0;
-    return carve(plan->d, max_rows, nullptr).total;
+    return carve(plan->d, plan->split_width, max_rows, nullptr).total;
 }
 
 int oco_moe_bind_workspace(oco_moe_plan* plan, void* workspace, size_t bytes, int max_rows) {
     if (!plan || !workspace || max_rows < 1) return fail(plan, OCO_INVALID_ARGUMENT, "null workspace or max_rows < 1");
     if (((uintptr_t)workspace & 255u) != 0) return fail(plan, OCO_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
-    Workspace ws = carve(plan->d, max_rows, (unsigned char*)workspace);
+    Workspace ws = carve(plan->d, plan->split_width, max_rows, (unsigned char*)workspace);
     if (bytes < ws.total) return fail(plan, OCO_INVALID_ARGUMENT, "workspace too small: %zu < %zu", bytes, ws.total);
     const oco_moe_desc& d = plan->d;
     // Control words and the never-written columns of the single-token fragments start at zero.
@@ -1129,7 +1129,6 @@ int oco_moe_bind_workspace(oco_moe_plan* plan, void* workspace, size_t bytes, in
     }
     if (d.shared_ffn) {
         CK(cudaMemset(ws.sh_actfrag, 0, (size_t)(d.shared_ffn / 32) * 128 * 2));
-        CK(cudaMemset(ws.sh_ids, 0, 256));
     }
     const uint64_t R = (uint64_t)max_rows * d.top_k;
     for (int i = 0; i < kTileKinds; i++) {
@@ -1676,6 +1675,7 @@ int oco_dense_plan_create(const oco_dense_desc* desc, oco_dense_plan** out) {
         return fail(dp->inner, OCO_UNSUPPORTED_SHAPE, "the relu^2 feed-forward is built for Q4_0 weights");
     if (desc->kind == OCO_DENSE_FFN_SILU_GATE && desc->weight_format != OCO_FMT_Q4_K)
         return fail(dp->inner, OCO_UNSUPPORTED_SHAPE, "the gated feed-forward is built for Q4_K weights");
+    if (split_tiles(dp->inner)) dp->inner->split_width = desc->kind == OCO_DENSE_PROJECTION ? desc->ffn : desc->hidden;
     return OCO_OK;
 }
 

@@ -41,8 +41,8 @@ struct DownDeal { int shares, turns, ksplit, sh_ksplit; };
 // narrow routes the proportion asks for more shares than there are CTAs. A unit of such a route is one or two blocks
 // long and costs its start, about a stage of 16 blocks. Hidden 4096, routes of 64, always-on expert of 4416, six routes:
 // 69 shares 78.5 us, 43 shares 43.1, five 32.9; hidden 2688, 32 and 4800: one share 41.1 us, 142 shares 54.6, ten 26.8.
-// For each number of turns only the largest
-// number of shares is looked at; it leaves the fewest CTAs idle. turns == 0: more places than CTAs.
+// For each number of turns only the largest number of shares is looked at; it leaves the fewest CTAs idle.
+// turns == 0: more places than CTAs.
 inline DownDeal deal_down(int K, int row_blocks, int nkb, int sh_nkb, int ctas, int warps_per_cta) {
     const int room = ctas - K;
     if (!sh_nkb || room < 1) {

@@ -116,3 +116,36 @@ def test_dense_window_and_graph_calls_check_their_arguments(lib):
     assert lib.oco_moe_experts_window(plan, None, None, 4, 1, 0, 0, 0, None, None) == _lib.INVALID_ARGUMENT
     assert lib.oco_moe_combine_shared(plan, None, None, None, None, 1, None) == _lib.INVALID_ARGUMENT
     lib.oco_moe_plan_destroy(plan)
+
+
+def test_only_plans_that_split_a_product_reserve_its_parts(lib, monkeypatch):
+    """Room for the f32 parts of a split dense product (148 CTAs of 256 x 256 at most) is there in a dense plan and in a
+    layer with an always-on expert, and nowhere else."""
+    rows, H = 512, 512
+
+    def moe_bytes(**kw):
+        rc, h, msg = _create(lib, **{**dict(arch=1, weight_format=2, hidden=H, ffn=H, experts=1, top_k=1), **kw})
+        assert rc == _lib.OK, msg
+        n = lib.oco_moe_workspace_bytes(h, rows)
+        lib.oco_moe_plan_destroy(h)
+        return n
+
+    def dense_bytes(kind, ffn=H):
+        d = _lib.DenseDesc(kind=kind, weight_format=2, hidden=H, ffn=ffn)
+        h = C.c_void_p()
+        assert lib.oco_dense_plan_create(C.byref(d), C.byref(h)) == _lib.OK
+        n = lib.oco_dense_workspace_bytes(h, rows)
+        lib.oco_dense_plan_destroy(h)
+        return n
+
+    parts = 148 // 2 * rows * H * 4            # two feature tiles of 256: 74 parts at most, and no more than 148 items hold
+    parts = min(parts, 148 * 256 * 256 * 4)
+    layer = moe_bytes()                        # a one-expert layer: routed products are never split
+    assert dense_bytes(0) == dense_bytes(1) == layer + parts
+    shared = moe_bytes(shared_ffn=64)
+    monkeypatch.setenv("OCO_MOE_NARROW_TILES", "1")
+    assert dense_bytes(0) == moe_bytes() == layer
+    assert shared == moe_bytes(shared_ffn=64) + parts
+    monkeypatch.delenv("OCO_MOE_NARROW_TILES")
+    assert moe_bytes(shared_ffn=64, gemm_impl=1) == shared - parts
+    assert dense_bytes(0, 19200) < moe_bytes(ffn=19200) + 256      # 75 feature tiles: more than half the CTAs, never split
