@@ -93,16 +93,16 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
     // ---- the work list ---------------------------------------------------------------------------
     const int nfeat = (p.n + kFeatPerItem - 1) / kFeatPerItem;
     const int ntiles = p.tiles ? (int)*p.tile_count : (p.dense_rows + NT - 1) / NT;
-    constexpr bool SPLIT = EPI == kEpiPartialF32;                      // the list runs once per part of the contraction
+    const int total = nfeat * ntiles;
+    // Split contraction: a CTA per item and part (launch_gemm_wide asks for total x splits of them), so a CTA's one item
+    // is the first it takes, over the K slices [kb0, kb1) of its part. Otherwise every item spans them all.
+    constexpr bool SPLIT = EPI == kEpiPartialF32;
     const int nkb = (p.K + 63) / 64;
-    const int total = nfeat * ntiles * (SPLIT ? p.splits : 1);
-    struct Item { uint32_t expert, row0, nv; int f0, kb0, kb1, split; };
+    const int part = SPLIT ? (int)blockIdx.x / total : 0, first_item = (int)blockIdx.x - part * total;
+    const int kb0 = SPLIT ? part * p.split_slices : 0, kb1 = SPLIT ? min(nkb, kb0 + p.split_slices) : nkb;
+    struct Item { uint32_t expert, row0, nv; int f0; };
     auto load_item = [&](int item) {
         Item r;
-        r.split = SPLIT ? item / (nfeat * ntiles) : 0;
-        r.kb0 = SPLIT ? r.split * p.split_slices : 0;
-        r.kb1 = SPLIT ? min(nkb, r.kb0 + p.split_slices) : nkb;
-        if (SPLIT) item -= r.split * nfeat * ntiles;
         const int tile = item / nfeat;
         r.f0 = (item - tile * nfeat) * kFeatPerItem;
         uint32_t begin, count;
@@ -173,8 +173,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         constexpr int NC = S::kCopies;
         constexpr uint32_t kBufBytes = 16 * S::kPitch;
         const uint32_t ring = ring_base + (uint32_t)warp * S::kRingWarp;
-        int chunk0 = 0, nchunks = (nkb + S::kChunkSlices - 1) / S::kChunkSlices;   // ring chunks [chunk0, nchunks) of an item
-        int g_run = 0;                                                         // slices of earlier items
+        const int chunk0 = kb0 / S::kChunkSlices, chunk1 = (kb1 + S::kChunkSlices - 1) / S::kChunkSlices;   // ring chunks of an item
         // packed bytes of tile row trow0 + r of an item
         auto row_ptr = [&](const Item& it, int r) -> const uint8_t* {
             const int feat0 = GATED ? it.f0 : it.f0 + 128 * tile;
@@ -191,7 +190,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
             cdst[i] = ring + (uint32_t)(crow[i] * S::kPitch + (idx % S::kRowChunks) * 16);
         }
         auto issue = [&](const uint8_t* const (&csrc)[NC], int chunk) {      // the K slices of ring chunk `chunk`
-            if (chunk < nchunks) {
+            if (chunk < chunk1) {
                 const uint32_t bsel = (uint32_t)(chunk & 1) * kBufBytes;
 #pragma unroll
                 for (int i = 0; i < NC; i++) {
@@ -223,33 +222,26 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         bool started = false;                 // the first ring buffer of `cur` is already on its way
         int seq = 0;
         const bool fetcher = warp == 0 && lane == 0;
-        if (fetcher) { item_slot[0] = blockIdx.x; mbar_arrive(item_full(0)); }
+        if (fetcher) { item_slot[0] = (uint32_t)first_item; mbar_arrive(item_full(0)); }
+        if (SPLIT && fetcher) { item_slot[1] = (uint32_t)total; mbar_arrive(item_full(1)); }   // there is no second one
         // the chunk during which the fetcher asks for the CTA's next item: late, so that a CTA holds no item it
         // will not start soon, yet a few slices before the end, so that the answer is there when the item ends
-        const int fetch_chunk = SPLIT ? -1 : max(0, nchunks - 4);
+        const int fetch_chunk = max(0, chunk1 - 4);
         uint32_t fetched = 0;
         int next = 0;
-        for (int item = blockIdx.x; item < total; item = next, seq++) {
+        for (int item = first_item; item < total; item = next, seq++) {
             if (!started) {
                 cur = load_item(item);
-                if (SPLIT) { chunk0 = cur.kb0 / S::kChunkSlices; nchunks = (cur.kb1 + S::kChunkSlices - 1) / S::kChunkSlices; }
 #pragma unroll
                 for (int i = 0; i < NC; i++) csrc[i] = row_ptr(cur, crow[i]);
                 issue(csrc, chunk0);
             }
             const uint32_t a_lo = (uint32_t)(uintptr_t)row_ptr(cur, r) & 15u;   // alignment of the row start
-            const int g0 = SPLIT ? g_run - cur.kb0 : seq * nkb;                  // slices of earlier items (less the first of this)
-            if (SPLIT) {
-                g_run += cur.kb1 - cur.kb0;
-                if (fetcher) {
-                    item_slot[(seq + 1) & 1] = min((uint32_t)item + gridDim.x, (uint32_t)total);
-                    mbar_arrive(item_full((seq + 1) & 1));
-                }
-            }
-            for (int chunk = chunk0; chunk < nchunks; chunk++) {
+            const int g0 = seq * (kb1 - kb0) - kb0;                              // slices of earlier items, less the first of this one
+            for (int chunk = chunk0; chunk < chunk1; chunk++) {
                 if (!SPLIT && fetcher) {
                     if (chunk == fetch_chunk) fetched = dyn ? gridDim.x + atomicAdd(p.sched, 1u) : (uint32_t)item + gridDim.x;
-                    if (chunk == min(fetch_chunk + 2, nchunks - 1)) {
+                    if (chunk == min(fetch_chunk + 2, chunk1 - 1)) {
                         item_slot[(seq + 1) & 1] = min(fetched, (uint32_t)total);
                         mbar_arrive(item_full((seq + 1) & 1));
                     }
@@ -272,7 +264,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
 #pragma unroll
                 for (int kk = 0; kk < S::kChunkSlices; kk++) {
                     const int kb = chunk * S::kChunkSlices + kk;
-                    if (kb < (SPLIT ? cur.kb1 : nkb)) {
+                    if (kb < kb1) {
                         uint32_t v[16];
                         if (SUPER) {
                             // code bytes 16 h .. 16 h + 15 of the slice's sub-block pair
@@ -320,7 +312,6 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
             started = next < total;
             if (started) {
                 cur = load_item(next);
-                if (SPLIT) { chunk0 = cur.kb0 / S::kChunkSlices; nchunks = (cur.kb1 + S::kChunkSlices - 1) / S::kChunkSlices; }
 #pragma unroll
                 for (int i = 0; i < NC; i++) csrc[i] = row_ptr(cur, crow[i]);
                 issue(csrc, chunk0);
@@ -357,7 +348,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     if (c + j < done.nv) {
-                        const size_t orow = ((SPLIT ? (size_t)done.split * p.dense_rows : 0) + out_rows[c + j]) * p.n;
+                        const size_t orow = ((SPLIT ? (size_t)part * p.dense_rows : 0) + out_rows[c + j]) * p.n;
                         const float a = __fadd_rn(__uint_as_float(ra[j]), bias_a);
                         const float b = __fadd_rn(__uint_as_float(rb[j]), bias_b);
                         if (SPLIT) {
@@ -381,7 +372,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
     } else if (warp == S::kMmaWarp) {
         if (lane == 0) {
             // ===== MMA issue ======================================================================
-            int seq = 0, g_run = 0;
+            int seq = 0;
             for (int item = item_of(0); item < total; item = item_of(++seq)) {
                 const Item it = load_item(item);
                 const uint32_t n_mma = max(16u, (it.nv + 15u) & ~15u);
@@ -390,9 +381,8 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                     mbar_wait(tmem_free, (uint32_t)(seq - 1) & 1u, abort_flag, p.status);
                     tc_fence_after();
                 }
-                const int g0 = SPLIT ? g_run - it.kb0 : seq * nkb;
-                if (SPLIT) g_run += it.kb1 - it.kb0;
-                for (int kb = it.kb0; kb < it.kb1; kb++) {
+                const int g0 = seq * (kb1 - kb0) - kb0;
+                for (int kb = kb0; kb < kb1; kb++) {
                     const int g = g0 + kb, sa = g % S::kAStages, sb = g % S::kBStages;
                     mbar_wait(full_a(sa), (uint32_t)(g / S::kAStages) & 1u, abort_flag, p.status);
                     mbar_wait(full_b(sb), (uint32_t)(g / S::kBStages) & 1u, abort_flag, p.status);
@@ -402,7 +392,7 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                     const uint64_t b = umma_desc(b_base + (uint32_t)sb * S::kBStage);
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
-                        const uint32_t acc = ((kb - it.kb0) | kk) != 0 ? 1u : 0u;
+                        const uint32_t acc = ((kb - kb0) | kk) != 0 ? 1u : 0u;
                         umma_f16(tmem_base, a0 + 2u * kk, b + 2u * kk, idesc, acc);
                         umma_f16(tmem_base + NT, a1 + 2u * kk, b + 2u * kk, idesc, acc);
                     }
@@ -416,15 +406,14 @@ grouped_gemm_wide_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         }
     } else if (lane == 0) {
         // ===== B tiles by TMA =========================================================================
-        int seq = 0, g_run = 0;
+        int seq = 0;
         for (int item = item_of(0); item < total; item = item_of(++seq)) {
             const Item it = load_item(item);
-            const int g0 = SPLIT ? g_run - it.kb0 : seq * nkb;
-            if (SPLIT) g_run += it.kb1 - it.kb0;
+            const int g0 = seq * (kb1 - kb0) - kb0;
             // the smallest box (32, 64, 128 or 256 rows of 64 halves) that holds the tile's live rows
             const CUtensorMap* box = it.nv <= 32 ? &tmap_b32 : it.nv <= 64 ? &tmap_b64 : it.nv <= 128 ? &tmap_b128 : &tmap_b;
             const uint32_t box_bytes = (it.nv <= 32 ? 32u : it.nv <= 64 ? 64u : it.nv <= 128 ? 128u : 256u) * 128u;
-            for (int kb = it.kb0; kb < it.kb1; kb++) {
+            for (int kb = kb0; kb < kb1; kb++) {
                 const int g = g0 + kb, sb = g % S::kBStages;
                 mbar_wait(empty_b(sb), ((uint32_t)(g / S::kBStages) & 1u) ^ 1u, abort_flag, p.status);
                 mbar_arrive_expect_tx(full_b(sb), box_bytes);
