@@ -34,7 +34,7 @@ def rel_l2(got_bits, ref_bits):
     return np.linalg.norm(g - r) / max(np.linalg.norm(r), 1e-30)
 
 
-def check(dense, oracle, kind, fmt, H, F, rows, seed, x_scale=1.0):
+def check(dense, oracle, kind, fmt, H, F, rows, seed, x_scale=1.0, launches=None):
     rng = np.random.default_rng(seed)
     gen = synth._RANDOM[fmt]
     up_w = gen(rng, F, H)
@@ -51,7 +51,7 @@ def check(dense, oracle, kind, fmt, H, F, rows, seed, x_scale=1.0):
     assert got.shape == ref.shape
     err = rel_l2(got, ref)
     assert err <= REL_L2, f"kind {kind} fmt {fmt} {H}x{F} rows {rows}: rel-L2 {err}"
-    assert plan.launch_count() >= 2
+    assert plan.launch_count() >= 2 if launches is None else plan.launch_count() == launches
     return got, ref, (up_w, gate_w, down_w, x_bits)
 
 
@@ -95,8 +95,15 @@ def test_mxfp4_projection_at_the_gpt_oss_width(dense, oracle):
                                           (synth.FMT_Q4_K, 7936, 32, 700), (synth.FMT_Q4_0, 8224, 64, 16)])
 def test_projection_over_a_split_contraction(dense, oracle, fmt, H, F, rows):
     """Few items and a long contraction: parts of unequal length, a last K slice that is half full, partial tiles of
-    features and rows. (Too short a contraction, or enough items, stays whole: the shapes above.)"""
-    check(dense, oracle, dense.PROJECTION, fmt, H, F, rows, 60 + rows, x_scale=0.25)
+    features and rows. (Too short a contraction, or enough items, stays whole: the shapes above.) Three launches: row conversion,
+    parts, sum."""
+    check(dense, oracle, dense.PROJECTION, fmt, H, F, rows, 60 + rows, x_scale=0.25, launches=3)
+
+
+@pytest.mark.parametrize("fmt,H,F,rows", [(synth.FMT_Q4_0, 320, 64, 300), (synth.FMT_MXFP4, 960, 19200, 20)], ids=["short", "many-items"])
+def test_projection_that_stays_whole(dense, oracle, fmt, H, F, rows):
+    """Too short a contraction, and more items than half the SMs: two launches."""
+    check(dense, oracle, dense.PROJECTION, fmt, H, F, rows, 60 + rows, x_scale=0.25, launches=2)
 
 
 def test_split_contraction_stores_to_any_output_address(dense, oracle):
@@ -114,6 +121,7 @@ def test_split_contraction_stores_to_any_output_address(dense, oracle):
         y = torch.full((rows * F + 2,), 77, dtype=torch.int16, device="cuda")
         plan.forward(x, y[skip:skip + rows * F], rows)
         torch.cuda.synchronize()
+        assert plan.launch_count() == 3
         assert bool((y[:skip] == 77).all()) and bool((y[skip + rows * F:] == 77).all())
         outs.append(y[skip:skip + rows * F].cpu().numpy())
     assert np.array_equal(outs[0], outs[1])
@@ -132,9 +140,11 @@ def test_a_step_after_a_wait_that_gave_up_leaves_the_output(dense, oracle, H, F,
     plan.bind(up_w, None, None)
     x_bits, _ = synth.make_tokens(H, rows, 6, "zero")
     x = torch.from_numpy(x_bits.view(np.int16)).cuda()
+    split = H > 1024
     y, again = (torch.full((rows, F), 77, dtype=torch.int16, device="cuda") for _ in range(2))
     plan.forward(x, y, rows)                       # leaves its parts in the workspace
     plan.poll()
+    assert plan.launch_count() == (3 if split else 2)
     want = y.clone()
     plan.workspace[:4].view(torch.int32).fill_(1)  # what a wait that gives up leaves there
     plan.forward(x, again, rows)

@@ -570,6 +570,18 @@ def test_few_tokens_tile_kernels(moe, oracle, monkeypatch, narrow):
         check_layer(moe, oracle, layer, tokens, seed=300 + tokens)
 
 
+@pytest.mark.parametrize("narrow", [False, True], ids=["wide", "generic"])
+@pytest.mark.parametrize("tokens", [2, 24])
+def test_qwen_few_tokens_tile_kernels(moe, oracle, monkeypatch, narrow, tokens):
+    """Thinly filled Q4_K tiles (32-row boxes, one or two live routes), which few tokens reach only when the streamed
+    kernels are switched off."""
+    monkeypatch.setenv("OCO_MOE_NO_BATCH", "1")
+    if narrow:
+        monkeypatch.setenv("OCO_MOE_NARROW_TILES", "1")
+    layer = synth.make_layer(synth.ARCH_QWEN, 512, 256, 128, 8, synth.FMT_Q4_K, seed=13)
+    check_layer(moe, oracle, layer, tokens, seed=300 + tokens)
+
+
 def test_gpt_oss_120b_decode_batch_full_size(moe, oracle):
     _sampled_full_size(moe, oracle, "gpt-oss-120b", 64, 4, seed=0, mode=2)
 
@@ -647,6 +659,23 @@ def test_interleaved_gate_up_is_bit_identical(moe, oracle, monkeypatch, tokens, 
         monkeypatch.setenv(k, v)
     layer = synth.make_layer(synth.ARCH_GPT_OSS, 320, 288, 8, 2, synth.FMT_MXFP4, seed=17)
     x, res = synth.make_tokens(320, tokens, 5, "normal")
+    split, r0 = moe.run_layer(layer, x, res, misalign=5)
+    both, r1 = moe.run_layer(layer, x, res, misalign=5, interleaved=True)
+    assert np.array_equal(split, both)
+    assert np.array_equal(r0["ids"], r1["ids"]) and np.array_equal(r0["y"], r1["y"])
+    ref = oracle.moe_forward(layer, x, res)
+    assert rel_l2(both, ref.out) <= REL_L2
+
+
+@pytest.mark.parametrize("tokens,env", [(1, {}), (6, {}), (40, {}), (40, {"OCO_MOE_NARROW_TILES": "1"}), (300, {})],
+                         ids=["t1", "t6", "t40", "t40-generic", "t300"])
+def test_interleaved_gate_up_q4_k(moe, oracle, monkeypatch, tokens, env):
+    """The same for Q4_K rows: single-token, streamed (six tokens) and tile kernels."""
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    layer = synth.make_layer(synth.ARCH_QWEN, 512, 256, 8, 2, synth.FMT_Q4_K, seed=19)
+    x, res = synth.make_tokens(512, tokens, 5, "normal")
+    x = synth.f32_to_bf16_bits(synth.bf16_bits_to_f32(x) * np.float32(0.125))      # keeps the half activations finite
     split, r0 = moe.run_layer(layer, x, res, misalign=5)
     both, r1 = moe.run_layer(layer, x, res, misalign=5, interleaved=True)
     assert np.array_equal(split, both)
