@@ -111,8 +111,15 @@ struct BatchParams {
 // (or fewer) the last wave decided: 19 groups made 152 CTAs of three rounds on 148 SMs, six rounds where three
 // suffice. Within its run a warp starts the next unit's first stage under the last stage of the one before, across
 // groups too, so that its rows never stop; only the group's fragments are waited for when the group changes.
-// gpt-oss-20b-shaped step of 7 tokens 156 -> 139 us (179 -> 139 with other routes), 120b-shaped one of 64 tokens 561 -> 492 us. Qwen3 (Q4_K), which
-// took 256-route tiles for any batch: 2 rows 136 -> 66 us, 8 rows 352 -> 130, 32 rows 254 -> 200, 96 rows 306 -> 250.
+// Up to 18 groups (eight CTAs and more each) whole rounds are too coarse: 15 groups of 180 units are 32 CTAs of two
+// rounds beside 116 of one. There the CTAs are dealt out to the groups and take equal shares of a group's units, unless
+// the longest share exceeds the longest run of whole rounds. With fewer CTAs to a group the equal runs are the better
+// deal: 8 to 20 tokens took 1 to 2 % longer with shares.
+// gpt-oss-20b-shaped layer, a CTA for each eighth | equal runs | this: 2 tokens 109.5 | 85.5 | 78.1 us, 5 tokens 113.4 | 118.8
+// | 112.7, 6 tokens 114.6 | 120.2 | 116.0, 8 tokens 187.6 | 136.2 | 136.1, 40 tokens 198 | 186 | 187; 7 tokens, norm
+// included, 130 or 153 by the routes | 131.6 | 128.7; 120b-shaped of 64 tokens 560 | 490 | 491 (519 | 487 on other routes).
+// Qwen3 (Q4_K), which took 256-route tiles for any batch: 2 rows 136 -> 66 us, 8 rows 351 -> 130, 32 rows 280 -> 210,
+// 96 rows 327 -> 259.
 template <int FMT, int EPI>
 __global__ void __launch_bounds__(kBatchThreads, 1) batch_rows_kernel(const BatchParams p) {
     constexpr bool GATED = epi_gated(EPI);
@@ -140,13 +147,24 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_rows_kernel(const Batc
     __syncthreads();          // the mbarriers exist
 
     const int units = p.n_out / ROWS, rounds = (units + kBatchWarps - 1) / kBatchWarps;
-    const long long total = (long long)*p.tile_count * rounds;
-    const int r_begin = (int)(total * blockIdx.x / gridDim.x), r_end = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    const int groups = (int)*p.tile_count, ctas = (int)gridDim.x, cta = (int)blockIdx.x, total = groups * rounds;   // total * ctas: well below 2^31
+    int r_begin = total * cta / ctas, r_end = total * (cta + 1) / ctas, first = warp, last = units;
+    const int per = groups ? ctas / groups : 0;
+    if (per >= 8 && (units + per - 1) / per <= kBatchWarps * ((total + ctas - 1) / ctas)) {
+        const int group = cta / per, k = cta - group * per;
+        r_begin = r_end = group * rounds;
+        if (group < groups) {                         // (the last CTAs may have no group)
+            first = units * k / per;
+            last = units * (k + 1) / per;
+            r_end += (last - first + kBatchWarps - 1) / kBatchWarps;
+            first += warp;
+        }
+    }
     // the spans of this warp's unit in a round; null where the group's last round has none for it
     auto spans = [&](int round, const uint8_t*& a, const uint8_t*& b) {
         a = b = nullptr;
-        const int group = round / rounds, u = (round - group * rounds) * kBatchWarps + warp;
-        if (u >= units) return;
+        const int group = round / rounds, u = (round - group * rounds) * kBatchWarps + first;
+        if (u >= last) return;
         const size_t off = ((size_t)__ldg(p.tiles + 2 * group) * p.n_out + (size_t)u * ROWS) * p.row_bytes;
         a = p.w0 + off;
         b = GATED ? p.w1 + off : a + (size_t)8 * p.row_bytes;
@@ -179,8 +197,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batch_rows_kernel(const Batc
         __half* fout = DOWN ? nullptr : p.frag_out + (size_t)group * (p.n_out / 32) * (kBatchFragBlock / 2);
         bool fetched = false;
         for (int round = r0; round < seg_end; round++) {
-            const int u = (round - group * rounds) * kBatchWarps + warp;
-            if (u >= units) continue;                 // na, nb stay: the unit of a later round
+            const int u = (round - group * rounds) * kBatchWarps + first;
+            if (u >= last) continue;                 // na, nb stay: the unit of a later round
             const uint8_t *a = na, *b = nb;
             find(round + 1);
             const int f0 = u * ROWS;

@@ -488,11 +488,13 @@ def test_nemotron_few_tokens_streamed(moe, oracle, tokens):
 
 @pytest.mark.parametrize("arch,hidden,ffn,experts,top_k,tokens",
                          [("gpt_oss", 96, 96, 32, 4, 3), ("gpt_oss", 288, 320, 32, 4, 64), ("gpt_oss", 640, 160, 128, 4, 250),
+                          ("gpt_oss", 640, 1120, 32, 4, 4), ("nemotron", 1056, 4000, 32, 2, 7),
                           ("nemotron", 256, 160, 128, 6, 90), ("nemotron", 96, 1056, 16, 2, 2), ("qwen", 256, 256, 16, 4, 2),
                           ("qwen", 512, 768, 128, 8, 9), ("qwen", 768, 512, 128, 8, 100)])
 def test_few_tokens_equal_shares(moe, oracle, arch, hidden, ffn, experts, top_k, tokens):
     """The persistent few-token kernel: fewer units than warps, a last round that some warps have no unit in, CTAs whose
-    run of rounds ends inside a group or spans several, fewer rounds than CTAs."""
+    run of rounds ends inside a group or spans several, fewer rounds than CTAs; equal shares of a group's units (few
+    groups) that end inside a round, CTAs left without a group."""
     if arch == "gpt_oss":
         layer = synth.make_layer(synth.ARCH_GPT_OSS, hidden, ffn, experts, top_k, synth.FMT_MXFP4, seed=hidden + ffn)
     elif arch == "qwen":
