@@ -812,42 +812,40 @@ int stage_experts(oco_moe_plan* plan, const uint16_t* x, const uint32_t* ids, in
         // A few routes per expert: memory-bound, streamed with up to eight routes per MMA (batch.cuh).
         // (Layers too wide for the fragments to sit in shared memory take the tiles, and so do rows that do not start on
         // eight bytes, which oco_moe_experts may be given: batch_fragments_kernel reads four values at once.)
-        {
-            plan->last_tile_rows = kBatchCols;
-            launch_route_plan(plan, ids, R, E, kBatchCols, rs, st);
-            const int groups = (int)batch_max_groups((size_t)R, (size_t)E);
-            mark(plan, st, "fragments");
-            CK(launch_dependent(batch_fragments_kernel<FMT>, dim3(groups), dim3(256), 0, st, x, ws.tiles, ws.tile_count, ws.offsets, ws.route_of_row, per_row,
-                                H, reinterpret_cast<uint4*>(ws.bfrag_in)));
-            plan->launches += 1;
-            // persistent: a CTA per SM, fewer where there are fewer rounds of sixteen 16-row units than SMs
-            const long long up_rounds = (F / (ARCH == OCO_ARCH_NEMOTRON ? 16 : 8) + kBatchWarps - 1) / kBatchWarps;
-            const long long down_rounds = (H / 16 + kBatchWarps - 1) / kBatchWarps;
-            const dim3 up_grid((unsigned)std::min<long long>(plan->sm_count, groups * up_rounds));
-            const dim3 down_grid((unsigned)std::min<long long>(plan->sm_count, groups * down_rounds));
-            ALLOW_SMEM_ONCE((batch_rows_kernel<FMT, EPI_UP>));
-            ALLOW_SMEM_ONCE((batch_rows_kernel<FMT, kEpiDownBf16>));
-            BatchParams bp{};
-            bp.tiles = ws.tiles; bp.tile_count = ws.tile_count; bp.offsets = ws.offsets; bp.route_of_row = ws.route_of_row;
-            bp.status = ws.status;
-            bp.w0 = ARCH == OCO_ARCH_NEMOTRON ? plan->up_rows : plan->gate_rows;
-            bp.w1 = ARCH == OCO_ARCH_NEMOTRON ? nullptr : plan->up_rows;
-            bp.b0 = ARCH == OCO_ARCH_GPT_OSS ? plan->gate_bias : nullptr;
-            bp.b1 = ARCH == OCO_ARCH_GPT_OSS ? plan->up_bias : nullptr;
-            bp.frag_in = ws.bfrag_in; bp.frag_out = ws.bfrag_out; bp.out = ws.act;
-            bp.n_in = H; bp.n_out = F; bp.row_bytes = plan->up_row_stride; bp.bias_stride = plan->up_bias_stride;
-            mark(plan, st, "up_rows");
-            CK(launch_dependent(batch_rows_kernel<FMT, EPI_UP>, up_grid, dim3(kBatchThreads), batch_smem_bytes(FMT, H / 32), st, bp));
-            bp.w0 = plan->w.down_w; bp.w1 = nullptr;
-            bp.b0 = ARCH == OCO_ARCH_GPT_OSS ? plan->w.down_b : nullptr; bp.b1 = nullptr;
-            bp.frag_in = ws.bfrag_out; bp.frag_out = nullptr; bp.out = y;
-            bp.n_in = F; bp.n_out = H; bp.row_bytes = plan->down_row_bytes; bp.bias_stride = 1;
-            mark(plan, st, "down_rows");
-            CK(launch_dependent(batch_rows_kernel<FMT, kEpiDownBf16>, down_grid, dim3(kBatchThreads), batch_smem_bytes(FMT, F / 32), st, bp));
-            plan->launches += 2;
-            CK(cudaGetLastError());
-            return OCO_OK;
-        }
+        plan->last_tile_rows = kBatchCols;
+        launch_route_plan(plan, ids, R, E, kBatchCols, rs, st);
+        const int groups = (int)batch_max_groups((size_t)R, (size_t)E);
+        mark(plan, st, "fragments");
+        CK(launch_dependent(batch_fragments_kernel<FMT>, dim3(groups), dim3(256), 0, st, x, ws.tiles, ws.tile_count, ws.offsets, ws.route_of_row, per_row,
+                            H, reinterpret_cast<uint4*>(ws.bfrag_in)));
+        plan->launches += 1;
+        // persistent: a CTA per SM, fewer where there are fewer rounds of sixteen 16-row units than SMs
+        const long long up_rounds = (F / (ARCH == OCO_ARCH_NEMOTRON ? 16 : 8) + kBatchWarps - 1) / kBatchWarps;
+        const long long down_rounds = (H / 16 + kBatchWarps - 1) / kBatchWarps;
+        const dim3 up_grid((unsigned)std::min<long long>(plan->sm_count, groups * up_rounds));
+        const dim3 down_grid((unsigned)std::min<long long>(plan->sm_count, groups * down_rounds));
+        ALLOW_SMEM_ONCE((batch_rows_kernel<FMT, EPI_UP>));
+        ALLOW_SMEM_ONCE((batch_rows_kernel<FMT, kEpiDownBf16>));
+        BatchParams bp{};
+        bp.tiles = ws.tiles; bp.tile_count = ws.tile_count; bp.offsets = ws.offsets; bp.route_of_row = ws.route_of_row;
+        bp.status = ws.status;
+        bp.w0 = ARCH == OCO_ARCH_NEMOTRON ? plan->up_rows : plan->gate_rows;
+        bp.w1 = ARCH == OCO_ARCH_NEMOTRON ? nullptr : plan->up_rows;
+        bp.b0 = ARCH == OCO_ARCH_GPT_OSS ? plan->gate_bias : nullptr;
+        bp.b1 = ARCH == OCO_ARCH_GPT_OSS ? plan->up_bias : nullptr;
+        bp.frag_in = ws.bfrag_in; bp.frag_out = ws.bfrag_out; bp.out = ws.act;
+        bp.n_in = H; bp.n_out = F; bp.row_bytes = plan->up_row_stride; bp.bias_stride = plan->up_bias_stride;
+        mark(plan, st, "up_rows");
+        CK(launch_dependent(batch_rows_kernel<FMT, EPI_UP>, up_grid, dim3(kBatchThreads), batch_smem_bytes(FMT, H / 32), st, bp));
+        bp.w0 = plan->w.down_w; bp.w1 = nullptr;
+        bp.b0 = ARCH == OCO_ARCH_GPT_OSS ? plan->w.down_b : nullptr; bp.b1 = nullptr;
+        bp.frag_in = ws.bfrag_out; bp.frag_out = nullptr; bp.out = y;
+        bp.n_in = F; bp.n_out = H; bp.row_bytes = plan->down_row_bytes; bp.bias_stride = 1;
+        mark(plan, st, "down_rows");
+        CK(launch_dependent(batch_rows_kernel<FMT, kEpiDownBf16>, down_grid, dim3(kBatchThreads), batch_smem_bytes(FMT, F / 32), st, bp));
+        plan->launches += 2;
+        CK(cudaGetLastError());
+        return OCO_OK;
     }
     if constexpr (ARCH == OCO_ARCH_GPT_OSS) {
         if (d.numerics == 2) return stage_experts_mx(plan, x, ids, R, per_row, y, st, rs);

@@ -715,7 +715,7 @@ struct DecodeDownParams {
 
 // Down products for one token: unit = 16 output rows of one route
 // (reference matvec_mxfp4, projections.metal:140-182; matvec_q4, vector.metal:155-228).
-// CTA c serves route c % K, so a CTA needs one route's fragments only.
+// CTA c serves place c % (K + sh_shares), a route or the always-on expert, so a CTA needs one set of fragments only.
 template <int FMT, int STAGES>
 __global__ void __launch_bounds__(tok_warps(FMT) * 32, 1) decode_down_kernel(const DecodeDownParams p) {
     constexpr int WARPS = tok_warps(FMT);
